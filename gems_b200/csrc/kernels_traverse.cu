@@ -1,4 +1,5 @@
-// kernels_traverse.cu -- whole-traversal kernels for 4- and 20-state models (FP64 and mixed).
+// kernels_traverse.cu -- whole-traversal kernels for 4-state models (FP64 and mixed) and the mixed
+// 20-state form on CUDA cores; the dispatch of both state counts (FP64, 20 states: kernels_f20.cu).
 //
 // One CTA owns a tile of patterns and runs every node update of the traversal over it, in
 // postorder; a pattern stays with one lane group for all ops, so a child written by an earlier
@@ -102,97 +103,8 @@ __global__ void k_prep_ops_f64(DevCtx c, const DevOp *ops, double *tab, size_t s
   for (int idx = threadIdx.x; idx < blk; idx += blockDim.x) leaf[rows + idx] = 1.0;
 }
 
-template <int N, bool SAFE>
-__device__ __forceinline__ void msg_f64(const DevCtx &c, const EigPack<N> &E, int kind, int id,
-                                        const double *__restrict__ d,
-                                        const double *__restrict__ leaf, long p, int gl,
-                                        double (&v)[N], int &s) {
-  const int C = c.C;
-  if (kind == GEMS_CHILD_TIP) {
-    const int st = min((int)c.tips[(size_t)id * c.P + p], c.unknown);
-    const double *lt = leaf + (size_t)st * c.block + gl;
-#pragma unroll
-    for (int x = 0; x < N; x++) v[x] = __ldg(lt + x * C);
-    s = 0;
-  } else {
-    double L[N];
-    load_row<N>(static_cast<const double *>(c.partials) + (size_t)id * c.slot_elems, c, p, gl, L);
-#pragma unroll
-    for (int i = 0; i < N; i++) L[i] *= __ldg(d + i * C + gl);
-#pragma unroll
-    for (int x = 0; x < N; x++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int i = 0; i < N; i++) acc = fma(E.evec[x * N + i], L[i], acc);
-      v[x] = acc;
-    }
-    const uint16_t *sc = c.scale + (size_t)id * c.slot_scale;
-    s = SAFE ? sc[(size_t)p * C + gl] : sc[p];
-  }
-}
-
-template <int N, bool SAFE>
-__global__ void __launch_bounds__(kThreads) k_traverse_f64(DevCtx c, const DevOp *__restrict__ ops,
-                                                           int nops,
-                                                           const double *__restrict__ tab,
-                                                           size_t stride, const EigPack<N> E,
-                                                           int p0, int p1) {
-  const int G = c.G;
-  const int gl = threadIdx.x & (G - 1);
-  const long p = p0 + ((long)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const bool act = p < p1 && gl < c.C;
-  const int C = c.C, blk = c.block;
-  double *part = static_cast<double *>(c.partials);
-  __shared__ int4 s_ops[kOpChunk];
-  for (int k = 0; k < nops; k++) {
-    if ((k & (kOpChunk - 1)) == 0) stage_ops(ops, k, nops, s_ops);
-    const OpIds op = staged_op(s_ops, k & (kOpChunk - 1));
-    const double *tk = tab + (size_t)k * stride;
-    const bool tiptip = op.l_kind == GEMS_CHILD_TIP && op.r_kind == GEMS_CHILD_TIP;
-    double out[N];
-    double lh_max = 0.0;
-    int sl = 0, sr = 0;
-    if (act) {
-      double tmp[N];
-      {
-        double vl[N], vr[N];
-        msg_f64<N, SAFE>(c, E, op.l_kind, op.l_id, tk, tk + 2 * blk, p, gl, vl, sl);
-        msg_f64<N, SAFE>(c, E, op.r_kind, op.r_id, tk + blk,
-                         tk + 2 * blk + (size_t)(c.unknown + 1) * blk, p, gl, vr, sr);
-#pragma unroll
-        for (int x = 0; x < N; x++) tmp[x] = vl[x] * vr[x];
-      }
-#pragma unroll
-      for (int j = 0; j < N; j++) {
-        double acc = 0.0;
-#pragma unroll
-        for (int x = 0; x < N; x++) acc = fma(E.inv[j * N + x], tmp[x], acc);
-        out[j] = acc;
-        lh_max = fmax(lh_max, fabs(acc));
-      }
-    }
-    if (!SAFE) lh_max = group_max(lh_max, G);
-    int s_out = sl + sr;
-    if (act) {
-      if (!tiptip && lh_max < kScaleThr && c.invar[p] == 0.0) {
-#pragma unroll
-        for (int j = 0; j < N; j++) out[j] = ldexp(out[j], kScaleExp);
-        s_out += 1;
-      }
-      store_row<N>(part + (size_t)op.dst_slot * c.slot_elems, c, p, gl, out);
-      uint16_t *sc = c.scale + (size_t)op.dst_slot * c.slot_scale;
-      if (SAFE)
-        sc[(size_t)p * C + gl] = (uint16_t)s_out;
-      else if (gl == 0)
-        sc[p] = (uint16_t)s_out;
-    }
-    __syncwarp();
-  }
-}
-
 // FP64, 4 states: PP patterns per lane group at B blocks per SM (as k_traverse_mix4), same
-// arithmetic in the same order as msg_f64 / k_traverse_f64, so every (PP, B) gives the same
-// values.  Measured on the 512-taxon, 1M-pattern case: one pattern per group (40 registers)
+// arithmetic in the same order, so every (PP, B) gives the same values.  Measured on the 512-taxon, 1M-pattern case: one pattern per group (40 registers)
 // 23.6 ms; two at 4 blocks per SM 22.5 ms, at 3 or 5 blocks 23.7 / 24.5 ms; three at 3 blocks
 // 22.4 ms; four at 2 blocks 24.7 ms.  The variant in use is picked by the tuner below.
 template <bool SAFE, int PP>
@@ -1653,9 +1565,8 @@ int traverse4(Session *s, bool mixed, int nops, int p0, int p1, const EigPack<4>
   return GEMS_OK;
 }
 
-template <int N>
-int launch_f64(Session *s, int nops, int p0, int p1) {
-  DevCtx c = s->ctx();
+int launch_f64_4(Session *s, int nops, int p0, int p1) {
+  constexpr int N = 4;
   EigPack<N> E;
   if (s->h_evec.size() != (size_t)N * N || s->h_inv.size() != (size_t)N * N) {
     set_error("eigensystem not set");
@@ -1665,21 +1576,7 @@ int launch_f64(Session *s, int nops, int p0, int p1) {
     E.evec[i] = s->h_evec[i];
     E.inv[i] = s->h_inv[i];
   }
-  const bool safe = s->desc.scaling == GEMS_SCALE_SAFE;
-  if constexpr (N == 4) {
-    return traverse4(s, false, nops, p0, p1, &E);
-  } else {
-    const int grid = grid_for(s, p0, p1);
-    if (safe)
-      k_traverse_f64<N, true><<<grid, kThreads, 0, s->stream>>>(c, s->d_ops, nops, s->d_opmats,
-                                                                 s->op_stride, E, p0, p1);
-    else
-      k_traverse_f64<N, false><<<grid, kThreads, 0, s->stream>>>(c, s->d_ops, nops, s->d_opmats,
-                                                                  s->op_stride, E, p0, p1);
-  }
-  s->launches++;
-  GEMS_CUDA(cudaGetLastError());
-  return GEMS_OK;
+  return traverse4(s, false, nops, p0, p1, &E);
 }
 
 }  // namespace
@@ -1690,6 +1587,8 @@ bool traverse_v2_supported(const Session *s) {
 
 int launch_prep_ops_v2(Session *s, int nops) {
   if (nops <= 0) return GEMS_OK;
+  if (s->desc.precision == GEMS_PREC_FP64 && s->desc.nstates == 20)
+    return launch_prep_ops_f20(s, nops);
   DevCtx c = s->ctx();
   if (s->desc.precision == GEMS_PREC_MIXED) {
     const size_t smem = sizeof(double) * s->block;
@@ -1727,9 +1626,10 @@ int traverse_v2_wave_patterns(const Session *s) {
     } else {
       return 0;
     }
+  } else if (mixed) {
+    fn = safe ? (const void *)k_traverse_mix<20, true> : (const void *)k_traverse_mix<20, false>;
   } else {
-    fn = mixed ? (safe ? (const void *)k_traverse_mix<20, true> : (const void *)k_traverse_mix<20, false>)
-               : (safe ? (const void *)k_traverse_f64<20, true> : (const void *)k_traverse_f64<20, false>);
+    fn = traverse_f20_kernel(s, &threads, &per_block);
   }
   int nsm = 0, per_sm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device) != cudaSuccess ||
@@ -1782,7 +1682,8 @@ int launch_traverse_v2(Session *s, int nops, int p0, int p1) {
       GEMS_CUDA(cudaGetLastError());
     }
   } else {
-    st = s->desc.nstates == 4 ? launch_f64<4>(s, nops, p0, p1) : launch_f64<20>(s, nops, p0, p1);
+    st = s->desc.nstates == 4 ? launch_f64_4(s, nops, p0, p1)
+                              : launch_traverse_f20(s, nops, p0, p1);
   }
   if (st) return st;
   return prof_end(s, 0, ev0);
