@@ -182,7 +182,10 @@ struct Session {
   double *d_red = nullptr;     // reduction partials
   double *d_result = nullptr;  // final scalars
   int *d_flag = nullptr;       // device status flags (barrier timeouts)
-  unsigned int *d_bar = nullptr;  // grid barrier counters
+  unsigned int *d_bar = nullptr;  // count of finished blocks of a branch-term launch (zero between)
+  void *d_slots = nullptr;        // the Newton kernel's exchange slots
+  unsigned int newton_launches = 0;
+  int newton_fit[2][2] = {{-1, -1}, {-1, -1}};  // clusters of 8, 16 the GPU holds, per kernel form
   // batched launches led by this session: job table (device and pinned host copies)
   static constexpr int kMaxBatch = 128;
   TcJob *d_jobs = nullptr;
@@ -250,15 +253,20 @@ int cuda_status(cudaError_t e, const char *what);
 int launch_prep_ops(Session *s, int nops);
 // patterns [p0, p1) of the traversal, p1 <= P (every launch_traverse* below alike)
 int launch_traverse(Session *s, int nops, int p0, int p1);
-int launch_branch_lnl(Session *s, const gems_branch *br, double *lnl);
-int launch_theta(Session *s, const gems_branch *br);
-int launch_derv(Session *s, double length, double *df, double *ddf);
+// branch terms (kernels_branch.cu).  theta_in_kernel: theta is formed by the kernel that uses it
+// (else launch it first: enqueue_theta_mixed); br null: theta as stored
+bool theta_in_kernel(const Session *s);
+// lnL or derivatives at `length`, theta kept with `store`; the results are in s->h_result once
+// the session's stream has completed (terms_lnl: the lnL of them)
+int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length);
+double terms_lnl(const Session *s);
+int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf);
 int launch_from_buffer(Session *s, double length, double *lnl);
-int launch_newton(Session *s, double length0, double min_len, double max_len, double xacc,
-                  int max_steps, double *opt_len, int *nevals);
-// the same in two halves: enqueue (result copied to pinned host memory), then wait and read
-int launch_newton_async(Session *s, double guess, double min_len, double max_len, double xacc,
-                        int max_steps);
+// the Newton loop in two halves: enqueue (result written to pinned host memory), then wait and
+// read
+size_t newton_slot_bytes();
+int launch_newton_async(Session *s, const gems_branch *br, double guess, double min_len,
+                        double max_len, double xacc, int max_steps);
 int newton_result(Session *s, double *opt_len, int *nevals);
 int launch_eigen(Session *s, const double *exch_upper, const double *freq);
 // the same for nsess sessions of one state count in one launch (inputs stacked per session)
@@ -267,12 +275,8 @@ int launch_eigen_batch(Session *const *ss, int nsess, const double *exch_upper,
 // mixed precision (kernels_mixed.cu)
 int launch_prep_ops_mixed(Session *s, int nops);
 int launch_traverse_mixed(Session *s, int nops, int p0, int p1);
-// the same without waiting: with want_lnl the result is copied to s->h_result, read by
-// theta_mixed_lnl once the session's stream has completed
+// theta of a 20- or 61-state branch, and with want_lnl its lnL (as enqueue_terms)
 int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta);
-double theta_mixed_lnl(const Session *s);
-int launch_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta,
-                       double *lnl);
 // factored whole-traversal kernels for 4 and 20 states (kernels_traverse.cu)
 bool traverse_v2_supported(const Session *s);
 int launch_prep_ops_v2(Session *s, int nops);

@@ -1,0 +1,919 @@
+// kernels_branch.cu -- the branch terms: log-likelihood, theta, derivatives, lnL from theta, and
+// the Newton loop on the device (phylokernelnew.h:2053-3495, utils/optimization.cpp:422-499).
+//
+// Every term is a dot product over the C * n elements of a pattern's theta = node (*) dad (eigen
+// space) with tables of exp(eval_i r_c t):
+//      lh = sum theta v0,   d1 = sum theta v1,   d2 = sum theta v2
+// so one layout serves all state counts: L lanes share a pattern (a power of two, at least C),
+// each lane taking a few element pairs (pair_of): a warp reads whole lines of the pattern-major
+// theta and partials whatever n is.  (One lane per category row, the form before, read n = 20 and 61
+// with a stride of n doubles: two to four times the sectors.)
+//
+// Theta is formed by the kernel that uses it, from the two partials, and stored for the calls
+// after it; the tables are computed by every block; the last block to finish adds the per-block
+// sums in index order and writes the result to pinned host memory.  One launch per call instead
+// of a table, a theta, a term and a reduction kernel and a copy: lnL and the derivatives of 29
+// branches of a 16-taxon, 3,801-pattern tree, bound by launches, take 0.93 ms instead of 1.29 ms;
+// the lnL of a 450,000-pattern tree from its partials and 256 replicates 141 us instead of 170.
+//
+// Reductions over patterns are deterministic: a fixed tree per block, then index order.
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <string>
+
+#include "gems_internal.cuh"
+#include "tc_common.cuh"
+
+namespace gems {
+
+namespace {
+
+// where theta comes from
+enum : int {
+  kMem = 0,  // c.theta
+  kT4,       // FP64 partials, 4 states (tile-major)
+  kR20,      // FP64 partials, 20 states (pattern-major)
+  kR61,      // FP64 partials, 61 states
+  kM4        // FP32 real-space partials, 4 states: lifted to the eigen basis in FP64
+};
+enum : int { kStore = 1, kLnl = 2, kDerv = 4 };
+
+template <int SRC>
+__host__ __device__ constexpr int src_states() {
+  return SRC == kR20 ? 20 : (SRC == kR61 ? 61 : 4);
+}
+
+// Lanes per pattern and pairs per lane for a block of B = C * n elements: at least C lanes (the
+// SAFE counters of a pattern, one per lane), more until a lane holds at most five pairs.
+struct Split {
+  int L, E2;
+};
+inline Split split_of(int B, int C) {
+  const int u = (B + 1) / 2;
+  int L = 2;
+  while (L < C) L *= 2;
+  while (L < 32 && (u + L - 1) / L > 5) L *= 2;
+  const int need = (u + L - 1) / L;
+  for (int e : {1, 2, 3, 4, 5, 8})
+    if (need <= e) return {L, e};
+  return {L, 16};  // 61 states, 16 categories: 488 pairs on 32 lanes
+}
+
+// the pair that lane l holds at q: strided, so that a warp reads whole lines, except for one or two
+// pairs per lane (4 states), where a lane holds a category's row (one 16- or 32-byte piece)
+template <int E2>
+__device__ __forceinline__ int pair_of(int q, int l, int L) {
+  return E2 <= 2 ? l * E2 + q : q * L + l;
+}
+
+// two elements j, j + 1 (j even) of a pattern-major row of `block` doubles
+__device__ __forceinline__ void row_pair(const double *row, int j, int block, double &a,
+                                         double &b) {
+  if (block % 2 == 0) {
+    const double2 v = __ldcg(reinterpret_cast<const double2 *>(row + j));
+    a = v.x, b = v.y;
+  } else {
+    a = __ldcg(row + j), b = j + 1 < block ? __ldcg(row + j + 1) : 0.0;
+  }
+}
+
+// elements i, i + 1 of inv_evec . v (4 states)
+__device__ __forceinline__ void lift2(const DevCtx &c, int i, float4 v, double &x, double &y) {
+  const double *r = c.inv_evec + i * 4;
+  auto row = [&](const double *q) {
+    double s = fma(__ldg(q), (double)v.x, 0.0);
+    s = fma(__ldg(q + 1), (double)v.y, s);
+    s = fma(__ldg(q + 2), (double)v.z, s);
+    return fma(__ldg(q + 3), (double)v.w, s);
+  };
+  x = row(r);
+  y = row(r + 4);
+}
+
+// This lane's theta elements of two patterns p[0], p[1], SAFE rows brought to the pattern's
+// smallest count (+1: times the scaling threshold, more: zero), and that count.  All loads are
+// issued before the first is used.  All lanes of a warp call it.
+template <int SRC, bool SAFE, int E2>
+__device__ __forceinline__ void load_theta(const DevCtx &c, const gems_branch &br, int L, int l,
+                                           const long (&p)[2], double (&th)[2][2 * E2],
+                                           int (&ms)[2]) {
+  constexpr int N = src_states<SRC>();
+  const bool act[2] = {p[0] < c.P, p[1] < c.P};
+  ms[0] = ms[1] = 0;
+  if constexpr (SRC == kMem) {
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int q = 0; q < E2; q++) {
+        const int j = 2 * pair_of<E2>(q, l, L);
+        th[u][2 * q] = th[u][2 * q + 1] = 0.0;
+        if (act[u] && j < c.block)
+          row_pair(c.theta + (size_t)p[u] * c.block, j, c.block, th[u][2 * q], th[u][2 * q + 1]);
+      }
+    return;
+  }
+  const bool is_tip = br.node_kind == GEMS_CHILD_TIP;
+  int tip[2] = {0, 0}, sd[2] = {0, 0}, sn[2] = {0, 0};
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    if (!act[u]) continue;
+    if (is_tip) tip[u] = c.tips[(size_t)br.node_id * c.P + p[u]];
+    if (!SAFE || l < c.C) {
+      const size_t o = SAFE ? (size_t)p[u] * c.C + l : (size_t)p[u];
+      sd[u] = c.scale[(size_t)br.dad_slot * c.slot_scale + o];
+      if (!is_tip) sn[u] = c.scale[(size_t)br.node_id * c.slot_scale + o];
+    }
+  }
+  if constexpr (SRC == kM4) {
+    const float *part = static_cast<const float *>(c.partials);
+    float4 d[2][E2], n[2][E2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int q = 0; q < E2; q++) {
+        const int j = 2 * pair_of<E2>(q, l, L);
+        d[u][q] = n[u][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // (two pairs: both of one category's row, which is read once)
+        if (!act[u] || j >= c.block || (E2 == 2 && q == 1)) continue;
+        const size_t o = mix_off<4>(c, p[u], j >> 2);
+        d[u][q] = __ldcg(reinterpret_cast<const float4 *>(part + (size_t)br.dad_slot * c.slot_elems + o));
+        if (!is_tip)
+          n[u][q] = __ldcg(reinterpret_cast<const float4 *>(part + (size_t)br.node_id * c.slot_elems + o));
+      }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int q = 0; q < E2; q++) {
+        const int i = 2 * pair_of<E2>(q, l, L) & 3, qq = E2 == 2 ? 0 : q;
+        double dx, dy, nx, ny;
+        lift2(c, i, d[u][qq], dx, dy);
+        if (is_tip) {
+          const double2 v = __ldg(reinterpret_cast<const double2 *>(c.tip + (size_t)tip[u] * 4 + i));
+          nx = v.x, ny = v.y;
+        } else {
+          lift2(c, i, n[u][qq], nx, ny);
+        }
+        th[u][2 * q] = nx * dx;
+        th[u][2 * q + 1] = ny * dy;
+      }
+  } else {
+    const double *part = static_cast<const double *>(c.partials);
+    const double *dad = part + (size_t)br.dad_slot * c.slot_elems;
+    const double *node = part + (size_t)br.node_id * c.slot_elems;
+    double n[2][2 * E2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int q = 0; q < E2; q++) {
+        const int j = 2 * pair_of<E2>(q, l, L);
+        double &a = th[u][2 * q], &b = th[u][2 * q + 1];
+        a = b = n[u][2 * q] = n[u][2 * q + 1] = 0.0;
+        if (!act[u] || j >= c.block) continue;
+        if constexpr (SRC == kT4) {
+          const size_t o = f64_off<4>(c, p[u], j >> 2, j & 3);
+          const double2 v = __ldcg(reinterpret_cast<const double2 *>(dad + o));
+          a = v.x, b = v.y;
+          if (!is_tip) {
+            const double2 w = __ldcg(reinterpret_cast<const double2 *>(node + o));
+            n[u][2 * q] = w.x, n[u][2 * q + 1] = w.y;
+          }
+        } else {
+          row_pair(dad + (size_t)p[u] * c.block, j, c.block, a, b);
+          if (!is_tip)
+            row_pair(node + (size_t)p[u] * c.block, j, c.block, n[u][2 * q], n[u][2 * q + 1]);
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int q = 0; q < E2; q++) {
+        if (is_tip) {
+          const int j = 2 * pair_of<E2>(q, l, L);
+          n[u][2 * q] = __ldg(c.tip + (size_t)tip[u] * N + j % N);
+          n[u][2 * q + 1] = __ldg(c.tip + (size_t)tip[u] * N + (j + 1) % N);
+        }
+        th[u][2 * q] *= n[u][2 * q];
+        th[u][2 * q + 1] *= n[u][2 * q + 1];
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int ss = sd[u] + sn[u];
+    ms[u] = ss;
+    if (!SAFE) continue;
+    if (!act[u] || l >= c.C) ms[u] = INT_MAX;
+    for (int o = 1; o < L; o <<= 1) ms[u] = min(ms[u], __shfl_xor_sync(0xffffffffu, ms[u], o));
+    if (!__any_sync(0xffffffffu, act[u] && l < c.C && ss != ms[u])) continue;
+    const double thr = SRC == kM4 ? 5.421010862427522e-20 /* 2^-64 */ : kScaleThr;
+    const int base = (threadIdx.x & 31) & ~(L - 1);
+#pragma unroll
+    for (int e = 0; e < 2 * E2; e++) {
+      const int j = 2 * pair_of<E2>(e >> 1, l, L) + (e & 1);
+      const int k = __shfl_sync(0xffffffffu, ss, base + min(j / N, c.C - 1));
+      if (k == ms[u] + 1)
+        th[u][e] *= thr;
+      else if (k > ms[u] + 1)
+        th[u][e] = 0.0;
+    }
+  }
+}
+
+template <int E2>
+__device__ __forceinline__ void store_theta(const DevCtx &c, int L, int l, long p,
+                                            const double (&th)[2 * E2]) {
+#pragma unroll
+  for (int q = 0; q < E2; q++) {
+    const int j = 2 * pair_of<E2>(q, l, L);
+    if (j >= c.block) continue;
+    double *d = c.theta + (size_t)p * c.block + j;
+    if (c.block % 2 == 0) {
+      *reinterpret_cast<double2 *>(d) = make_double2(th[2 * q], th[2 * q + 1]);
+    } else {
+      d[0] = th[2 * q];
+      if (j + 1 < c.block) d[1] = th[2 * q + 1];
+    }
+  }
+}
+
+// eval_i r_c and prop_c of element j of the block (zero past it)
+__device__ __forceinline__ void table_factors(const DevCtx &c, int j, double &cof, double &prop) {
+  cof = prop = 0.0;
+  if (j < c.block) {
+    const int cc = j / c.n, i = j - cc * c.n;
+    cof = c.eval[i] * c.rates[cc];
+    prop = c.props[cc];
+  }
+}
+// v0 = exp(eval_i r_c t) prop_c, v1 = (eval_i r_c) v0, v2 = (eval_i r_c) v1 (`len` elements each,
+// nt tables)
+__device__ __forceinline__ void put_tables(double t, int j, double cof, double prop, int len,
+                                           int nt, double *v) {
+  const double a = exp(cof * t) * prop, b = cof * a;
+  v[j] = a;
+  if (nt > 1) {
+    v[len + j] = b;
+    v[2 * len + j] = cof * b;
+  }
+}
+
+// dot product of this lane's elements with a table, then the sum over the pattern's lanes
+template <int E2>
+__device__ __forceinline__ double dot(const double (&th)[2 * E2], const double *v, int L, int l) {
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < E2; q++) {
+    const double2 w = *reinterpret_cast<const double2 *>(v + 2 * pair_of<E2>(q, l, L));
+    s = fma(w.x, th[2 * q], s);
+    s = fma(w.y, th[2 * q + 1], s);
+  }
+  return s;
+}
+// x of the first pattern, y of the second: even lanes end with x's sum over the pattern's lanes,
+// odd lanes with y's (one exchange fewer than two sums)
+__device__ __forceinline__ double lanes_sum2(double x, double y, int L, int l) {
+  const double keep = l & 1 ? y : x, give = l & 1 ? x : y;
+  double s = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+  for (int o = 2; o < L; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// sums of two values over the block in a fixed tree; valid in the first warp's lane 0
+template <int NW>
+__device__ __forceinline__ void block_pair(double &a, double &b, double (*sh)[2]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) sh[w][0] = a, sh[w][1] = b;
+  __syncthreads();
+  if (w == 0) {
+    a = lane < NW ? sh[lane][0] : 0.0;
+    b = lane < NW ? sh[lane][1] : 0.0;
+    for (int o = NW / 2; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+  }
+}
+
+constexpr int kThreadsT = 256;
+// resident blocks per SM (the registers of two patterns' elements)
+constexpr int ctas_t(int e2) { return e2 <= 2 ? 3 : (e2 <= 5 ? 2 : 1); }
+
+// One evaluation at length t: flags kStore (theta and scale_all kept), kLnl (pattern_lh; out =
+// lnL, lnL with non-finite patterns clamped) or kDerv (df_frac, ddf_term; out = df, ddf).
+template <int SRC, bool SAFE, int E2>
+__global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
+    k_terms(DevCtx c, gems_branch br, double t, int L, int flags, unsigned int *ticket,
+            double *out) {
+  extern __shared__ __align__(16) double tab[];
+  __shared__ double sh[kThreadsT / 32][2];
+  __shared__ bool last;
+  const int len = 2 * L * E2;
+  for (int j = threadIdx.x; j < len; j += kThreadsT) {
+    double cof, prop;
+    table_factors(c, j, cof, prop);
+    put_tables(t, j, cof, prop, len, flags & kDerv ? 3 : 1, tab);
+  }
+  __syncthreads();
+  const int l = threadIdx.x & (L - 1);
+  const long per = blockDim.x / L, step = per * gridDim.x;
+  double v0 = 0.0, v1 = 0.0;
+  constexpr double thr = SRC == kM4 ? kLogScaleThrF : kLogScaleThr;
+  // two patterns at a time: their loads overlap, and the logarithm or the division of the first
+  // is the even lanes', of the second the odd lanes'
+  for (long b = (long)blockIdx.x * per; b < c.P; b += 2 * step) {
+    const long pu[2] = {b + threadIdx.x / L, b + step + threadIdx.x / L};
+    const long p = l & 1 ? pu[1] : pu[0];
+    double th[2][2 * E2], iv = 0.0, f = 0.0, sc = 0.0;
+    int ms[2];
+    if (l < 2 && p < c.P) {
+      iv = c.invar[p];
+      f = c.freq[p];
+      if (SRC == kMem && (flags & kLnl)) sc = c.scale_all[p];
+    }
+    load_theta<SRC, SAFE, E2>(c, br, L, l, pu, th, ms);
+    if (flags & kStore) {
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        if (pu[u] < c.P) {
+          store_theta<E2>(c, L, l, pu[u], th[u]);
+          if (l == 0) c.scale_all[pu[u]] = (double)ms[u] * thr;
+        }
+    }
+    const double lh = lanes_sum2(dot<E2>(th[0], tab, L, l), dot<E2>(th[1], tab, L, l), L, l);
+    double d1 = 0.0, d2 = 0.0;
+    if (flags & kDerv) {
+      const double *t1 = tab + len, *t2 = t1 + len;
+      d1 = lanes_sum2(dot<E2>(th[0], t1, L, l), dot<E2>(th[1], t1, L, l), L, l);
+      d2 = lanes_sum2(dot<E2>(th[0], t2, L, l), dot<E2>(th[1], t2, L, l), L, l);
+    }
+    if (l >= 2 || p >= c.P) continue;
+    const double like = fabs(lh) + iv;
+    if (flags & kDerv) {
+      if (p >= c.nptn) continue;
+      const double inv = 1.0 / like;
+      const double dff = d1 * inv, ddff = d2 * inv;
+      const double t1 = dff * f, t2 = ddff * f;
+      v0 += t1;
+      v1 += fma(-t1, dff, t2);
+      c.df_frac[p] = dff;
+      c.ddf_term[p] = fma(-dff, dff, ddff);
+    } else {
+      const double plh = log(like) + (SRC == kMem ? sc : (l ? ms[1] : ms[0]) * thr);
+      c.pattern_lh[p] = plh;
+      if (p < c.nptn) {
+        v0 += plh * f;
+        v1 += (isfinite(plh) ? plh : 4.0 * kLogScaleThr) * f;
+      }
+    }
+  }
+  block_pair<kThreadsT / 32>(v0, v1, sh);
+  if (threadIdx.x == 0) {
+    __stcg(c.red + 2 * blockIdx.x, v0);
+    __stcg(c.red + 2 * blockIdx.x + 1, v1);
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v0 = v1 = 0.0;
+  for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+    v0 += __ldcg(c.red + 2 * b);
+    v1 += __ldcg(c.red + 2 * b + 1);
+  }
+  __syncthreads();
+  block_pair<kThreadsT / 32>(v0, v1, sh);
+  if (threadIdx.x == 0) {
+    out[0] = v0;
+    out[1] = v1;
+    *ticket = 0;  // ready for the next launch
+  }
+}
+
+// ----------------------------------------------------------------------------------------
+// Device-side Newton (Optimization::minimizeNewton) as one launch.  Each evaluation is a sum of
+// (df, ddf) over all patterns; every thread then runs the same scalar update on the same sums, so
+// all follow one iterate sequence.  A thread keeps its first patterns' theta in registers over
+// all evaluations, the others are read again each time.
+//
+// An evaluation is a chain of latencies (exponentials, dot products, sums over lanes, warps and
+// blocks, one division), so the exchange between blocks is what its design is about:
+// - Within a cluster, every warp sends its sums to each block's shared memory (st.async, counted
+//   by that block's mbarrier), and every warp adds all of them in one order: no barrier of the
+//   block, no leader, no broadcast.  Up to 16 blocks (8,192 patterns of 4 states and 4
+//   categories) need nothing else.
+// - Beyond that, each cluster of 8 publishes its sums in global memory, each with a tag (launch
+//   number, evaluation) in one 16-byte store, and the first warp of every block polls all
+//   clusters' slots until they carry the tag: one trip through L2.  Tags of earlier launches
+//   never match, so nothing is cleared.  Two sets of slots (and of shared-memory buffers) in
+//   turn: a set is written again only by who has seen everyone's next sums, which each sends
+//   after reading this set.
+// Every wait is bounded; who gives up sends nothing more, so the others give up too, and all
+// reach the cluster barrier at the end.
+// Measured, a loop of five evaluations (theta of 4,703 / 18,501 patterns of 4 states, 9,707 of 20,
+// 4 categories): 31.1 / 37.2 / 47.8 us with a counting barrier over 74 / 290 / 152 blocks and a
+// theta launch of 4.8 / 4.5 / 9.6 us before it; 28.9 / 39.7 / 46.3 us, theta included, with an
+// all-to-all exchange of every block's sums through L2 (4,000 to 7,200 cycles of an evaluation);
+// 25.6 / 27.0 / 32.1 us, theta included, as here.
+// ----------------------------------------------------------------------------------------
+constexpr int kPollLimit = 1 << 20;  // each poll is an L2 round trip or two: a second or so
+constexpr int kMaxClusters = 32;
+constexpr int kMaxCluster = 16;
+
+__device__ __forceinline__ void publish(ulonglong2 *slot, double v, unsigned long long tag) {
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\tmov.b128 r, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], r;\n\t}\n" ::"l"(
+          slot),
+      "l"(__double_as_longlong(v)), "l"(tag)
+      : "memory");
+}
+__device__ __forceinline__ bool peek(const ulonglong2 *slot, unsigned long long tag, double &v) {
+  unsigned long long a, b;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\tld.relaxed.gpu.global.b128 r, [%2];\n\tmov.b128 {%0, %1}, r;\n\t}\n"
+      : "=l"(a), "=l"(b)
+      : "l"(slot)
+      : "memory");
+  v = __longlong_as_double(a);
+  return b == tag;
+}
+
+// Sums of n <= 32 published pairs (slot pairs 128 bytes apart), by one warp: the same bits in
+// every lane of every caller; false when they have not all come in time.
+constexpr int kSlotStride = 8;  // ulonglong2 per pair
+__device__ __forceinline__ bool gather(const ulonglong2 *slots, int n, unsigned long long tag,
+                                       double &a, double &b) {
+  const int lane = threadIdx.x & 31;
+  bool ok = false;
+  for (int k = 0; k < kPollLimit && !ok; k++) {
+    a = b = 0.0;
+    bool mine = true;
+    if (lane < n) {
+      const bool u = peek(slots + kSlotStride * lane, tag, a);
+      const bool v = peek(slots + kSlotStride * lane + 1, tag, b);
+      mine = u && v;
+    }
+    ok = __all_sync(0xffffffffu, mine);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  return ok;
+}
+
+// The exchange's time-out path on purpose: each block publishes and waits for one more than
+// there are, so it gives up after kPollLimit polls and the flag reads GEMS_ERR_TIMEOUT.
+__global__ void k_exchange_probe(ulonglong2 *slots, int *flag) {
+  if (threadIdx.x == 0) {
+    publish(slots + kSlotStride * blockIdx.x, 1.0, 1);
+    publish(slots + kSlotStride * blockIdx.x + 1, 2.0, 1);
+  }
+  double a, b;
+  const bool ok = gather(slots, gridDim.x + 1, 1, a, b);
+  if (threadIdx.x == 0) atomicExch(flag, ok ? GEMS_OK : GEMS_ERR_TIMEOUT);
+}
+
+// address of this CTA's shared-memory location in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send_pair(uint32_t dst, uint32_t bar, double a, double b) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+      "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(bar)
+      : "memory");
+}
+
+struct NewtonArgs {
+  gems_branch br;
+  double guess, x1, x2, xacc;
+  int maxstep, L, cluster;   // blocks per cluster
+  ulonglong2 *slots;         // two sets of kMaxClusters pairs
+  unsigned long long tag0;   // launch number, shifted
+  double *result;            // pinned host memory: length, evaluations, status
+};
+
+// threads per block: more than five pairs per lane need more than 128 registers
+__host__ __device__ constexpr int newton_threads(int e2) { return e2 <= 5 ? 512 : 256; }
+template <int E2>
+__host__ __device__ constexpr int held_rows() {
+  return E2 <= 2 ? 4 : 2;  // an even number
+}
+
+template <int SRC, bool SAFE, int E2>
+__global__ void __launch_bounds__(newton_threads(E2), 1)
+    k_newton(DevCtx c, const NewtonArgs a) {
+  constexpr int kThreadsN = newton_threads(E2), kWarps = kThreadsN / 32;
+  extern __shared__ __align__(16) double tab[];
+  __shared__ __align__(16) double2 recv[2][kMaxCluster * kWarps];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ double tot[2];
+  __shared__ bool tot_ok;
+  constexpr int RH = held_rows<E2>();
+  constexpr double thr = SRC == kM4 ? kLogScaleThrF : kLogScaleThr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int CS = a.cluster, nclusters = gridDim.x / CS, rank = blockIdx.x % CS;
+  const int L = a.L, len = 2 * L * E2, l = threadIdx.x & (L - 1);
+  const long per = kThreadsN / L, step = per * gridDim.x;
+  const long b0 = (long)blockIdx.x * per;
+  const int sub = threadIdx.x / L;
+  const uint32_t s_recv = tc::sptr(&recv[0][0]), s_bars = tc::sptr(&bars[0]);
+  const uint32_t expect = CS * kWarps * sizeof(double2);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; i++) {
+      tc::mbar_init(s_bars + 8 * i, 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < 2; i++) tc::mbar_expect_tx(s_bars + 8 * i, expect);
+  }
+  // the others' barriers are ready once all blocks have been here (waited for below)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+
+  // theta of this thread's rows: formed and stored (or read), the first ones kept; of each two
+  // patterns, even lanes hold the first's +I term and weight and odd lanes the second's
+  double th[RH][2 * E2], inva[RH / 2], fr[RH / 2];
+  auto weights = [&](long p, double &iv, double &f) {
+    iv = f = 0.0;
+    if (l < 2 && p < c.nptn) iv = c.invar[p], f = c.freq[p];
+  };
+  auto keep = [&](const long (&p)[2], const double (&v)[2][2 * E2], const int (&m)[2]) {
+    if (SRC == kMem) return;
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (p[u] < c.P) {
+        store_theta<E2>(c, L, l, p[u], v[u]);
+        if (l == 0) c.scale_all[p[u]] = (double)m[u] * thr;
+      }
+  };
+#pragma unroll
+  for (int r = 0; r < RH; r += 2) {
+    const long p[2] = {b0 + r * step + sub, b0 + (r + 1) * step + sub};
+    inva[r / 2] = fr[r / 2] = 0.0;
+#pragma unroll
+    for (int e = 0; e < 2 * E2; e++) th[r][e] = th[r + 1][e] = 0.0;
+    if (b0 + r * step >= c.P) continue;
+    double v[2][2 * E2];
+    int m[2];
+    weights(l & 1 ? p[1] : p[0], inva[r / 2], fr[r / 2]);
+    load_theta<SRC, SAFE, E2>(c, a.br, L, l, p, v, m);
+    keep(p, v, m);
+#pragma unroll
+    for (int e = 0; e < 2 * E2; e++) th[r][e] = v[0][e], th[r + 1][e] = v[1][e];
+  }
+  if (SRC != kMem)
+    for (long b = b0 + RH * step; b < c.P; b += 2 * step) {
+      const long p[2] = {b + sub, b + step + sub};
+      double v[2][2 * E2];
+      int m[2];
+      load_theta<SRC, SAFE, E2>(c, a.br, L, l, p, v, m);
+      keep(p, v, m);
+    }
+
+  // this thread's table elements (at most 2 x 32 x E2 of them)
+  constexpr int kTab = (64 * E2 + kThreadsN - 1) / kThreadsN;
+  double cof[kTab], prop[kTab];
+#pragma unroll
+  for (int i = 0; i < kTab; i++) table_factors(c, threadIdx.x + i * kThreadsN, cof[i], prop[i]);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+
+  int nevals = 0;
+  // f = -dlnL/dt and df = -d2lnL/dt2 at t (computeFuncDerv, phylotree.cpp:2555).  Tables of the
+  // last evaluation may be overwritten: its sums have come, so every warp had read them.
+  auto eval = [&](double t, double &f, double &df) -> bool {
+#pragma unroll
+    for (int i = 0; i < kTab; i++)
+      if (threadIdx.x + i * kThreadsN < len)
+        put_tables(t, threadIdx.x + i * kThreadsN, cof[i], prop[i], len, 3, tab);
+    __syncthreads();
+    double v0 = 0.0, v1 = 0.0;
+    // two patterns' terms, b and b + step from this block's start
+    auto add = [&](const double (&x)[2 * E2], const double (&y)[2 * E2], long b, double iv,
+                   double w) {
+      const double *t1 = tab + len, *t2 = t1 + len;
+      const double h = lanes_sum2(dot<E2>(x, tab, L, l), dot<E2>(y, tab, L, l), L, l);
+      const double d = lanes_sum2(dot<E2>(x, t1, L, l), dot<E2>(y, t1, L, l), L, l);
+      const double g = lanes_sum2(dot<E2>(x, t2, L, l), dot<E2>(y, t2, L, l), L, l);
+      if (l < 2 && b + l * step + sub < c.nptn) {
+        const double inv = 1.0 / (fabs(h) + iv);
+        const double dff = d * inv, q = dff * w;
+        v0 += q;
+        v1 += fma(-q, dff, g * inv * w);
+      }
+    };
+#pragma unroll
+    for (int r = 0; r < RH; r += 2)
+      if (b0 + r * step < c.P) add(th[r], th[r + 1], b0 + r * step, inva[r / 2], fr[r / 2]);
+    for (long b = b0 + RH * step; b < c.P; b += 2 * step) {
+      const long p[2] = {b + sub, b + step + sub};
+      double v[2][2 * E2], iv, w;
+      int m[2];
+      weights(l & 1 ? p[1] : p[0], iv, w);
+      load_theta<kMem, SAFE, E2>(c, a.br, L, l, p, v, m);
+      add(v[0], v[1], b, iv, w);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    const int set = nevals & 1, use = (nevals >> 1) & 1;  // buffers; how often they were used, mod 2
+    nevals++;
+    const uint32_t bar = s_bars + 8 * set;
+    if (lane < CS)
+      send_pair(cluster_addr(s_recv + (set * kMaxCluster * kWarps + rank * kWarps + warp) * 16, lane),
+                cluster_addr(bar, lane), v0, v1);
+    bool ok = tc::mbar_wait(bar, use);
+    v0 = v1 = 0.0;
+    if (ok)
+      for (int i = lane; i < CS * kWarps; i += 32) {
+        const double2 v = recv[set][i];
+        v0 += v.x;
+        v1 += v.y;
+      }
+    // armed again for the evaluation after next, whose sums are sent after this one's were read
+    if (threadIdx.x == 0 && ok) tc::mbar_expect_tx(bar, expect);
+    for (int o = 16; o > 0; o >>= 1) {
+      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (nclusters > 1) {
+      if (warp == 0) {
+        ulonglong2 *slots = a.slots + set * kMaxClusters * kSlotStride;
+        const unsigned long long tag = a.tag0 + (unsigned)nevals;
+        if (ok && rank == 0 && lane < 2)
+          publish(slots + kSlotStride * (blockIdx.x / CS) + lane, lane ? v1 : v0, tag);
+        ok = gather(slots, nclusters, tag, v0, v1) && ok;
+        if (lane == 0) tot[0] = v0, tot[1] = v1, tot_ok = ok;
+      }
+      __syncthreads();
+      v0 = tot[0];
+      v1 = tot[1];
+      ok = tot_ok;
+    } else {
+      ok = __syncthreads_and(ok);
+    }
+    if (!ok) return false;
+    if (!isfinite(v0)) v0 = v1 = 0.0;
+    f = -v0;
+    df = -v1;
+    return true;
+  };
+
+  const double x1 = a.x1, x2 = a.x2, xacc = a.xacc;
+  double f, df, dx, temp, xh, xl, rts, rts_old;
+  double ret = 0.0;
+  int status = GEMS_OK;
+  rts = a.guess;
+  if (rts < x1) rts = x1;
+  if (rts > x2) rts = x2;
+  do {
+    if (!eval(rts, f, df)) { status = GEMS_ERR_TIMEOUT; ret = rts; break; }
+    if (!isfinite(f) || !isfinite(df)) { status = GEMS_ERR_NUMERIC_UNDERFLOW; ret = rts; break; }
+    if (df >= 0.0 && fabs(f) < xacc) { ret = rts; break; }
+    if (f < 0.0) { xl = rts; xh = x2; } else { xh = rts; xl = x1; }
+    dx = fabs(xh - xl);
+    bool done = false;
+    for (int j = 1; j <= a.maxstep && !done; j++) {
+      rts_old = rts;
+      const double newton = f / df;  // beside the bracket test, not after it
+      if ((df <= 0.0) || (((rts - xh) * df - f) * ((rts - xl) * df - f) >= 0.0)) {
+        dx = 0.5 * (xh - xl);
+        rts = xl + dx;
+        if (xl == rts) { ret = rts; done = true; break; }
+      } else {
+        dx = newton;
+        temp = rts;
+        rts -= dx;
+        if (temp == rts) { ret = rts; done = true; break; }
+      }
+      if (fabs(dx) < xacc || (j == a.maxstep)) { ret = rts_old; done = true; break; }
+      if (!eval(rts, f, df)) { status = GEMS_ERR_TIMEOUT; ret = rts; done = true; break; }
+      if (!isfinite(f) || !isfinite(df)) {
+        status = GEMS_ERR_NUMERIC_UNDERFLOW; ret = rts; done = true; break;
+      }
+      if (df > 0.0 && fabs(f) < xacc) { ret = rts; done = true; break; }
+      if (f < 0.0) xl = rts;
+      else if (f > 0.0) xh = rts;
+    }
+    if (!done) ret = 0.0;
+  } while (false);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.result[0] = ret;
+    a.result[1] = (double)nevals;
+    a.result[2] = (double)status;
+  }
+  // no block leaves while another may still send to its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ---- kernel tables -------------------------------------------------------------------------
+struct Fns {
+  const void *terms, *newton;
+};
+template <int SRC, bool SAFE, int E2>
+Fns fns() {
+  return {(const void *)k_terms<SRC, SAFE, E2>, (const void *)k_newton<SRC, SAFE, E2>};
+}
+template <int SRC, bool SAFE>
+Fns pick4(int e2) {  // 4 states: one or two pairs per lane
+  return e2 == 1 ? fns<SRC, SAFE, 1>() : fns<SRC, SAFE, 2>();
+}
+template <int SRC, bool SAFE>
+Fns pick(int e2) {  // the pairs per lane that split_of gives for 20 and 61 states
+  if (e2 <= 3) return fns<SRC, SAFE, 3>();
+  if (e2 == 4) return fns<SRC, SAFE, 4>();
+  if constexpr (SRC == kR61) {
+    if (e2 == 8) return fns<SRC, SAFE, 8>();
+    if (e2 == 16) return fns<SRC, SAFE, 16>();
+  }
+  return fns<SRC, SAFE, 5>();
+}
+Fns pick_mem(int e2) {
+  switch (e2) {
+    case 1: return fns<kMem, false, 1>();
+    case 2: return fns<kMem, false, 2>();
+    case 3: return fns<kMem, false, 3>();
+    case 4: return fns<kMem, false, 4>();
+    case 5: return fns<kMem, false, 5>();
+    case 8: return fns<kMem, false, 8>();
+    default: return fns<kMem, false, 16>();
+  }
+}
+Fns kernels_for(const Session *s, bool from_partials, int e2) {
+  const bool safe = s->desc.scaling == GEMS_SCALE_SAFE;
+  if (!from_partials) return pick_mem(e2);
+  if (s->desc.precision == GEMS_PREC_MIXED)
+    return safe ? pick4<kM4, true>(e2) : pick4<kM4, false>(e2);
+  switch (s->desc.nstates) {
+    case 4: return safe ? pick4<kT4, true>(e2) : pick4<kT4, false>(e2);
+    case 20: return safe ? pick<kR20, true>(e2) : pick<kR20, false>(e2);
+    default: return safe ? pick<kR61, true>(e2) : pick<kR61, false>(e2);
+  }
+}
+
+}  // namespace
+
+bool theta_in_kernel(const Session *s) {
+  return s->desc.precision == GEMS_PREC_FP64 || s->desc.nstates == 4;
+}
+
+// br: theta from the branch's partials; null: theta as stored.  The two results are in
+// s->h_result once the stream has completed.
+int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length) {
+  DevCtx c = s->ctx();
+  Split sp = split_of(s->block, s->desc.ncat);
+  const Fns f = kernels_for(s, br != nullptr, sp.E2);
+  const long per = kThreadsT / sp.L;
+  const int grid = (int)std::min<long>(148 * ctas_t(sp.E2), (s->P + per - 1) / per);
+  gems_branch b{};
+  if (br) b = *br;
+  int flags = (store ? kStore : 0) | (lnl ? kLnl : kDerv);
+  const size_t smem = sizeof(double) * 2 * sp.L * sp.E2 * (lnl ? 1 : 3);
+  unsigned int *ticket = s->d_bar;
+  double *out = s->h_result;
+  void *args[] = {&c, &b, &length, &sp.L, &flags, &ticket, &out};
+  const int id = lnl ? (br ? 1 : 4) : 3;
+  cudaEvent_t ev0;
+  if (int st = prof_begin(s, id, &ev0)) return st;
+  GEMS_CUDA(cudaLaunchKernel(f.terms, dim3(grid), dim3(kThreadsT), args, smem, s->stream));
+  s->launches++;
+  return prof_end(s, id, ev0);
+}
+
+// a non-finite total: the sum with non-finite pattern values clamped to 4 log(2^-256)
+// (phylokernelnew.h:3168-3184)
+double terms_lnl(const Session *s) {
+  return std::isfinite(s->h_result[0]) ? s->h_result[0] : s->h_result[1];
+}
+
+int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf) {
+  if (int st = enqueue_terms(s, br, br != nullptr, false, length)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  *df = s->h_result[0];
+  *ddf = s->h_result[1];
+  if (!std::isfinite(*df)) *df = *ddf = 0.0;  // phylokernelnew.h:2646-2649
+  return GEMS_OK;
+}
+
+int launch_from_buffer(Session *s, double length, double *lnl) {
+  if (int st = enqueue_terms(s, nullptr, false, true, length)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  *lnl = terms_lnl(s);
+  return GEMS_OK;
+}
+
+size_t newton_slot_bytes() { return sizeof(ulonglong2) * 2 * kMaxClusters * kSlotStride; }
+
+int newton_result(Session *s, double *opt_len, int *nevals) {
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  *opt_len = s->h_result[0];
+  *nevals = (int)s->h_result[1];
+  return (int)s->h_result[2];
+}
+
+int launch_newton_async(Session *s, const gems_branch *br, double guess, double min_len,
+                        double max_len, double xacc, int max_steps) {
+  DevCtx c = s->ctx();
+  const Split sp = split_of(s->block, s->desc.ncat);
+  const Fns f = kernels_for(s, br != nullptr, sp.E2);
+  int nsm = 0;
+  GEMS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device));
+  const size_t smem = sizeof(double) * 2 * sp.L * sp.E2 * 3;
+  const int threads = newton_threads(sp.E2);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeCooperative;  // all clusters of a launch resident together
+  attr[1].val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->stream;
+  cfg.attrs = attr;
+  // One block per SM at most, two patterns a thread where that fills them (a pair costs little
+  // more than one): one cluster of up to 16 blocks, which also holds up to the register rows of
+  // its threads, else clusters of 8, as many as the GPU takes at once.
+  const long per = threads / sp.L, held = sp.E2 <= 2 ? 4 : 2;
+  const int most = std::max(1, nsm / s->newton_share);
+  const long want = (s->P + 2 * per - 1) / (2 * per);
+  int *fits = s->newton_fit[br != nullptr];
+  auto fit = [&](int size) {  // clusters of 8 or 16 that the GPU holds at once
+    int &n = fits[size == 16];
+    if (n >= 0) return n;
+    if (size == 16 && cudaFuncSetAttribute(f.newton, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                           1) != cudaSuccess) {
+      cudaGetLastError();
+      return n = 0;
+    }
+    attr[0].val.clusterDim.x = size;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(size);
+    int m = 0;
+    if (cudaOccupancyMaxActiveClusters(&m, f.newton, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      m = 0;
+    }
+    return n = m;
+  };
+  const int one = most >= 16 && fit(16) > 0 ? 16 : 8;  // the largest single cluster
+  int cluster = 1, clusters = 1;
+  if (s->P <= one * per * held || most < 16 || fit(8) < 2) {
+    while (cluster < want && 2 * cluster <= std::min(most, one)) cluster *= 2;
+  } else {
+    cluster = 8;
+    clusters = (int)std::min<long>({(want + 7) / 8, most / 8, fit(8), kMaxClusters});
+  }
+  attr[0].val.clusterDim.x = cluster;
+  cfg.numAttrs = clusters > 1 ? 2 : 1;
+  cfg.gridDim = dim3(cluster * clusters);
+  NewtonArgs a{};
+  if (br) a.br = *br;
+  a.guess = guess;
+  a.x1 = min_len;
+  a.x2 = max_len;
+  a.xacc = xacc;
+  a.maxstep = max_steps;
+  a.L = sp.L;
+  a.cluster = cluster;
+  a.slots = reinterpret_cast<ulonglong2 *>(s->d_slots);
+  a.tag0 = (unsigned long long)(++s->newton_launches) << 32;
+  a.result = s->h_result;
+  void *args[] = {&c, &a};
+  cudaEvent_t ev0;
+  if (int st = prof_begin(s, 5, &ev0)) return st;
+  GEMS_CUDA(cudaLaunchKernelExC(&cfg, f.newton, args));
+  s->launches++;
+  return prof_end(s, 5, ev0);
+}
+
+int check_barrier_timeout(int device, int *status) {
+  GEMS_CUDA(cudaSetDevice(device));
+  ulonglong2 *slots = nullptr;
+  int *flag = nullptr;
+  GEMS_CUDA(cudaMalloc((void **)&slots, newton_slot_bytes()));
+  cudaError_t e = cudaMalloc((void **)&flag, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(slots, 0, newton_slot_bytes());
+  if (e == cudaSuccess) e = cudaMemset(flag, 0, sizeof(int));
+  if (e == cudaSuccess) {
+    void *args[] = {&slots, &flag};
+    e = cudaLaunchCooperativeKernel((void *)k_exchange_probe, dim3(2), dim3(32), args, 0, nullptr);
+  }
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  int h = -1;
+  if (e == cudaSuccess) e = cudaMemcpy(&h, flag, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(slots);
+  cudaFree(flag);
+  if (e != cudaSuccess) return cuda_status(e, "exchange probe");
+  *status = h;
+  return GEMS_OK;
+}
+
+}  // namespace gems

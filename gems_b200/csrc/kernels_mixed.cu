@@ -372,7 +372,7 @@ int launch_traverse_mixed(Session *s, int nops, int p0, int p1) {
   return prof_end(s, 0, ev0);
 }
 
-// theta (and optionally the branch lnL) from the two FP32 partials of br
+// theta (and optionally the branch lnL) from the two FP32 partials of br, 20 or 61 states
 int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta) {
   DevCtx c = s->ctx();
   const int grid = grid_for(s);
@@ -385,9 +385,9 @@ int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool s
   cudaEvent_t ev0;
   if (int st = prof_begin(s, want_lnl ? 1 : 2, &ev0)) return st;
   const int wl = want_lnl ? 1 : 0, stt = store_theta ? 1 : 0;
-  GEMS_DISPATCH_NM(s->desc.nstates, "theta_mixed",
-    if (safe) k_theta_mixed<NS, true><<<grid, kThreads, 0, s->stream>>>(c, *br, wl, stt, val);
-    else k_theta_mixed<NS, false><<<grid, kThreads, 0, s->stream>>>(c, *br, wl, stt, val));
+  auto *fn = s->desc.nstates == 20 ? (safe ? k_theta_mixed<20, true> : k_theta_mixed<20, false>)
+                                   : (safe ? k_theta_mixed<61, true> : k_theta_mixed<61, false>);
+  fn<<<grid, kThreads, 0, s->stream>>>(c, *br, wl, stt, val);
   s->launches++;
   GEMS_CUDA(cudaGetLastError());
   if (int st = prof_end(s, want_lnl ? 1 : 2, ev0)) return st;
@@ -397,19 +397,6 @@ int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool s
   GEMS_CUDA(cudaGetLastError());
   GEMS_CUDA(cudaMemcpyAsync(s->h_result, s->d_result, 2 * sizeof(double), cudaMemcpyDeviceToHost,
                             s->stream));
-  return GEMS_OK;
-}
-
-double theta_mixed_lnl(const Session *s) {
-  return std::isfinite(s->h_result[0]) ? s->h_result[0] : s->h_result[1];
-}
-
-int launch_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta,
-                       double *lnl) {
-  if (int st = enqueue_theta_mixed(s, br, want_lnl, store_theta)) return st;
-  if (!want_lnl) return GEMS_OK;
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
-  *lnl = theta_mixed_lnl(s);
   return GEMS_OK;
 }
 

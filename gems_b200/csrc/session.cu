@@ -193,6 +193,7 @@ static void free_session(Session *s) {
   cudaFree(s->d_result);
   cudaFree(s->d_flag);
   cudaFree(s->d_bar);
+  cudaFree(s->d_slots);
   cudaFreeHost(s->h_ops);
   cudaFree(s->d_jobs);
   cudaFreeHost(s->h_jobs);
@@ -347,6 +348,18 @@ static void copy_pattern_lh(Session *s, double *pattern_lh, double lnl_raw_finit
     if (!std::isfinite(pattern_lh[p])) pattern_lh[p] = 4.0 * kLogScaleThr;
 }
 
+// the lnL of a branch from its partials
+static int enqueue_branch_lnl(Session *s, const gems_branch *br) {
+  if (theta_in_kernel(s)) return enqueue_terms(s, br, false, true, br->length);
+  return enqueue_theta_mixed(s, br, true, false);
+}
+static int launch_branch_lnl(Session *s, const gems_branch *br, double *lnl) {
+  if (int st = enqueue_branch_lnl(s, br)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  *lnl = terms_lnl(s);
+  return GEMS_OK;
+}
+
 // largest state byte of the uploaded tips in columns [c0, c1) (rows of P bytes, P a multiple of
 // 64, the first nptn of each row valid; c0 and c1 multiples of 16): a grid-stride loop over
 // 16-byte words, per-byte maxima with __vmaxu4
@@ -487,6 +500,7 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
   ALLOC(s->d_result, 16 * sizeof(double));
   ALLOC(s->d_flag, 16 * sizeof(int));
   ALLOC(s->d_bar, 16 * sizeof(unsigned int));
+  ALLOC(s->d_slots, newton_slot_bytes());
 #undef ALLOC
   if ((e = cudaHostAlloc((void **)&s->h_ops, (size_t)z.nops_max * sizeof(DevOp), 0)) !=
       cudaSuccess)
@@ -505,6 +519,8 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
       (e = cudaMemsetAsync(s->d_freq, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_invar, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_scale, 0, z.scale_bytes, s->stream)) ||
+      (e = cudaMemsetAsync(s->d_bar, 0, 16 * sizeof(unsigned int), s->stream)) ||
+      (e = cudaMemsetAsync(s->d_slots, 0, newton_slot_bytes(), s->stream)) ||
       (e = cudaStreamSynchronize(s->stream)))
     return fail(e, "initialise session");
   *out = s;
@@ -858,19 +874,12 @@ int gems_branch_lnl_batch_ops(gems_session *const *ss, int nsess, const gems_op 
     if (ss[i])
       if (int st = check_branch(ss[i], &br[i])) return st;
   if (int st = traverse_batch_lists(ss, nsess, ops, nops)) return st;
-  bool mixed = true;
-  for (int i = 0; i < nsess; i++) mixed = mixed && ss[i]->desc.precision == GEMS_PREC_MIXED;
-  if (!mixed) {
-    for (int i = 0; i < nsess; i++)
-      if (int st = gems_branch_lnl(ss[i], nullptr, 0, &br[i], &lnl[i], nullptr)) return st;
-    return GEMS_OK;
-  }
   // every session's branch terms enqueued on its own stream first, then the results read
   for (int i = 0; i < nsess; i++)
-    if (int st = enqueue_theta_mixed(ss[i], &br[i], true, false)) return st;
+    if (int st = enqueue_branch_lnl(ss[i], &br[i])) return st;
   for (int i = 0; i < nsess; i++) {
     GEMS_CUDA(cudaStreamSynchronize(ss[i]->stream));
-    lnl[i] = theta_mixed_lnl(ss[i]);
+    lnl[i] = terms_lnl(ss[i]);
   }
   return GEMS_OK;
 }
@@ -891,11 +900,7 @@ int gems_branch_lnl(gems_session *s, const gems_op *ops, int nops, const gems_br
   int st = check_branch(s, br);
   if (st) return st;
   if ((st = run_ops(s, ops, nops))) return st;
-  if (s->desc.precision == GEMS_PREC_MIXED)
-    st = launch_theta_mixed(s, br, true, false, lnl);
-  else
-    st = launch_branch_lnl(s, br, lnl);
-  if (st) return st;
+  if ((st = launch_branch_lnl(s, br, lnl))) return st;
   copy_pattern_lh(s, pattern_lh, *lnl);
   return GEMS_OK;
 }
@@ -991,9 +996,7 @@ int gems_branch_lnl_from_host(gems_session *s, const uint8_t *states, const doub
   }
   s->tips_ok = true;
   invalidate_theta(s, ops, nops);
-  st = s->desc.precision == GEMS_PREC_MIXED ? launch_theta_mixed(s, br, true, false, lnl)
-                                            : launch_branch_lnl(s, br, lnl);
-  if (st) return st;
+  if ((st = launch_branch_lnl(s, br, lnl))) return st;
   copy_pattern_lh(s, pattern_lh, *lnl);
   return GEMS_OK;
 }
@@ -1006,16 +1009,15 @@ int gems_branch_derv(gems_session *s, const gems_op *ops, int nops, const gems_b
   if (st) return st;
   if (compute_theta) {
     if ((st = run_ops(s, ops, nops))) return st;
-    st = s->desc.precision == GEMS_PREC_MIXED ? launch_theta_mixed(s, br, false, true, nullptr)
-                                              : launch_theta(s, br);
-    if (st) return st;
+    if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
     s->theta_valid = true;
     s->theta_branch = *br;
   } else if (!s->theta_valid) {
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
-  if ((st = launch_derv(s, br->length, df, ddf))) return st;
+  const bool form = compute_theta && theta_in_kernel(s);
+  if ((st = launch_derv(s, form ? br : nullptr, br->length, df, ddf))) return st;
   if (df_frac) {
     GEMS_CUDA(cudaMemcpyAsync(df_frac, s->d_df_frac, sizeof(double) * s->desc.nptn,
                               cudaMemcpyDeviceToHost, s->stream));
@@ -1047,16 +1049,15 @@ int gems_newton_branch_async(gems_session *s, const gems_op *ops, int nops,
   if (st) return st;
   if (compute_theta) {
     if ((st = run_ops(s, ops, nops))) return st;
-    st = s->desc.precision == GEMS_PREC_MIXED ? launch_theta_mixed(s, br, false, true, nullptr)
-                                              : launch_theta(s, br);
-    if (st) return st;
+    if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
     s->theta_valid = true;
     s->theta_branch = *br;
   } else if (!s->theta_valid) {
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
-  return launch_newton_async(s, br->length, min_len, max_len, xacc, max_steps);
+  return launch_newton_async(s, compute_theta && theta_in_kernel(s) ? br : nullptr, br->length,
+                             min_len, max_len, xacc, max_steps);
 }
 
 int gems_newton_branch_wait(gems_session *s, double *opt_len, int *nevals) {
