@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
     }
     if (!SAFE && act && t == 0)
       c.scale[(size_t)op.dst_slot * c.slot_scale + p] = (uint16_t)s_norm;
+    __syncwarp();  // the counters lane t = 0 wrote are read by its pattern's four lanes
     op = nxt;
     tl = tip_byte(op.l_kind, op.l_id);
     tr = tip_byte(op.r_kind, op.r_id);

@@ -11,24 +11,22 @@
 // a 160-taxon tree with long branches it moved partials by up to 2.5e-8 of their pattern's
 // largest value, measured in plain FP64 numpy as well.)
 //
-// Two kernels share the per-op tables (prep) and the row layout of the partial slots:
-// - k_traverse_g61m (SAFE scaling): the GEMMs on the FP64 tensor cores (mma.sync m8n8k4 f64),
-//   one CTA per tile of 64 patterns of ONE category -- categories are independent under SAFE
-//   scaling -- so that a CTA reads one E table per side and op (32 KB) instead of C of them;
+// - k_traverse_g61w (SAFE scaling, the usual one for 61 states): warps of 8 patterns of one
+//   category with chained products on the FP64 mma (below).
 // - k_traverse_g61 (NORM scaling, whose per-pattern maximum spans the categories): FP64 FMA,
 //   one CTA per tile of up to 64 rows = tp patterns x C categories (tp = 64 / C rounded down to
 //   a multiple of 8), stored category-major (row = c * tp + pattern), 128 threads as 8 x 16:
 //   thread (ty, tx) owns rows ty*8..ty*8+7 -- all of one category -- and columns tx, tx+16,
-//   tx+32, tx+48 (32 FP64 accumulators).
-// Both: two CTAs per SM, so that one's loads overlap the other's GEMMs; the A operand of a child
-// (its partial rows) staged k-major in shared memory; inv_evec^T in shared memory for the whole
-// traversal; E_c^T read through L1 from the op table (stored [side][c][k][64 columns] by the
-// prep kernel) and prefetched into L1 while the child's rows load.  A tip child's V is a row of
-// the op's leaf table (E_c . tip vector), gathered by state.  The tensor-core products come out
-// bit-identical to the FMA ones (the tests compare every partial).  Measured on one 200-taxon
-// codon model (3,780 patterns): per-row kernel 26.6 ms (+G4); FMA tiles of 128 rows 7.0 ms, with
-// the L1 prefetch 5.9 ms, 64-row tiles at two CTAs per SM 5.3 ms; tensor cores with mixed
-// categories per tile 5.9 ms (spills), one category per tile 4.7 ms (+R8: 11.9 -> 9.6 ms).
+//   tx+32, tx+48 (32 FP64 accumulators); two CTAs per SM; the A operand of a child (its partial
+//   rows) staged k-major in shared memory, inv_evec^T there for the whole traversal, E_c^T read
+//   through L1 from the op table ([side][c][k][64 columns]) and prefetched into L1 while the
+//   child's rows load; a tip child's V is a row of the op's leaf table, gathered by state.
+// The mma sums come out bit-identical to the FMA ones (the tests compare every partial).
+// Measured on one 200-taxon codon model (3,780 patterns, +G4), a from-scratch traversal: per-row
+// kernel 26.6 ms; FMA tiles of 128 rows 7.0 ms, with the L1 prefetch 5.9 ms, 64-row tiles at two
+// CTAs per SM 5.3 ms; mma over rows staged in shared memory between products 4.7 ms; chained in
+// registers 2.4 ms.  lnL and eight branch derivatives of that model: 11.6 -> 5.0 ms with the last
+// form, its op tables (mma as well, 17 us where one thread per element took 234) included.
 #include <string>
 
 #include "gems_internal.cuh"
@@ -123,20 +121,6 @@ struct TileMap {
   __device__ bool valid(int r) const { return r < nrow && pattern(r) < P; }
   // offset of the row's first state in the slot
   __device__ size_t off(int r) const { return ((size_t)pattern(r) * C + cat(r)) * kN; }
-};
-
-// SAFE only: a tile of 64 patterns of one category (categories are independent under SAFE
-// scaling), so a CTA reads one E table per side instead of C
-struct TileMap1 {
-  int C, tp, nrow, c0;
-  long p0, P;
-  __device__ int cat(int) const { return c0; }
-  __device__ long pattern(int r) const { return p0 + r; }
-  __device__ bool valid(int r) const { return p0 + r < P; }
-  __device__ size_t off(int r) const { return ((size_t)(p0 + r) * C + c0) * kN; }
-  __device__ int tile_row(int g) const { return g < kRows ? g : -1; }
-  __device__ bool row_ok(int g) const { return g < kRows && p0 + g < P; }
-  __device__ size_t slot_row(int g) const { return (size_t)(p0 + g) * C + c0; }
 };
 
 // V of one child for the thread's rows and columns, and its scale counts (per row: SAFE; the
@@ -308,193 +292,233 @@ __global__ void __launch_bounds__(kThreadsG, 2)
 }
 
 // ---------------------------------------------------------------------------------------
-// The same traversal with the GEMMs on the FP64 tensor cores (mma.sync m8n8k4 f64: one warp
-// instruction does 8 x 8 x 4 multiply-adds).  Warp w owns rows 16w..16w+15 as two 8-row blocks
-// (each of one category, tp being a multiple of 8) and all 64 columns as eight 8-column blocks;
-// lane l holds rows l/4 and columns 2(l%4), 2(l%4)+1 of each 8 x 8 block (the instruction's
-// accumulator layout).  Operand rows in shared memory are 72 doubles apart, so that the four
-// k-rows of a fragment load fall in two bank halves.
+// SAFE scaling: categories are independent, so a CTA owns 64 patterns of ONE category and its
+// warps 8 patterns each, for the whole op list, with the products on the FP64 mma (m8n8k4).
+//
+// Lane (g, t) = (lane / 4, lane % 4) holds A[g][k = t], B[k = t][n = g] and C[g][2t], C[g][2t + 1].
+// K step s covers states 4s .. 4s + 3 (the sums run in index order, as in the per-row kernel);
+// column n = 2 t' + e of N tile m stands for state 8m + 4e + t', so lane t's C fragment of a
+// product holds states 4s + t, s = 2m + e: the A fragments of the next one.  Products chain in
+// registers, a lane always holds the states {4s + t} of pattern g (it stores and re-reads those
+// elements itself: no synchronisation between ops), and the child that the last op wrote comes
+// from registers (the plan's forward bit).
+//
+// Both operands' B fragments lie in shared memory in lane order (one 16-byte read gives two):
+// inv_evec for the whole traversal, E_c of the next two internal children in a ring of two 32 KB
+// slots filled by cp.async while the product before runs; one barrier per product.
+// Bound by FP64 throughput: 256 mma per 8 patterns and op with one internal child.
 // ---------------------------------------------------------------------------------------
-constexpr int kLdM = 72;
-constexpr size_t kSmemM = sizeof(double) * 2 * (size_t)kK * kLdM;
+constexpr int kFrag = kK * kNC;               // doubles of one matrix in fragment order
+constexpr int kWarpsW = 8, kThreadsW = 32 * kWarpsW;
+constexpr size_t kSmemW = sizeof(double) * 3 * (size_t)kFrag;
+static_assert(kWarpsW * 8 == kRows, "a warp holds 8 patterns");
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
 }
-
-// acc[rb][cb] = A[rows of row block rb][k] . B_rb[k][columns of block cb] over k < kK, with
-// A k-major in shared memory (row stride kLdM) and B_rb = B0 or B1 (row stride ldb)
-template <bool GLOBAL_B>
-__device__ __forceinline__ void gemm_mma(const double *__restrict__ sA,
-                                         const double *__restrict__ B0,
-                                         const double *__restrict__ B1, int ldb, int w, int lane,
-                                         double (&acc)[2][8][2]) {
+// element i of a matrix in fragment order, [16 K steps][4 pairs of N tiles][32 lanes][2]: its
+// contraction index k and output state x
+__device__ __forceinline__ void frag_place(int i, int &k, int &x) {
+  const int lane = (i >> 1) & 31, m = 2 * ((i >> 6) & 3) + (i & 1), n = lane >> 2;
+  k = 4 * (i >> 8) + (lane & 3);
+  x = 8 * m + 4 * (n & 1) + (n >> 1);
+}
+// v <- M . v for the warp's 8 patterns
+__device__ __forceinline__ void product(const double *frag, int lane, double (&v)[16]) {
+  __syncwarp();
+  double acc[8][2];
 #pragma unroll
-  for (int rb = 0; rb < 2; rb++)
+  for (int m = 0; m < 8; m++) acc[m][0] = acc[m][1] = 0.0;
+  const double2 *f = reinterpret_cast<const double2 *>(frag) + lane;
 #pragma unroll
-    for (int cb = 0; cb < 8; cb++) acc[rb][cb][0] = acc[rb][cb][1] = 0.0;
-  const int kr = lane & 3, rc = lane >> 2;
-  const bool same = B0 == B1;
-#pragma unroll 2
-  for (int k0 = 0; k0 < kK; k0 += 4) {
-    const double *ar = sA + (k0 + kr) * kLdM + 16 * w + rc;
-    const double a0 = ar[0], a1 = ar[8];
-    const double *b0 = B0 + (size_t)(k0 + kr) * ldb + rc;
-    double bv[8];
+  for (int s = 0; s < 16; s++) {
+    double2 b[4];
 #pragma unroll
-    for (int cb = 0; cb < 8; cb++) bv[cb] = GLOBAL_B ? __ldg(b0 + 8 * cb) : b0[8 * cb];
+    for (int q = 0; q < 4; q++) b[q] = f[(s * 4 + q) * 32];
 #pragma unroll
-    for (int cb = 0; cb < 8; cb++) dmma(acc[0][cb], a0, bv[cb]);
-    if (same) {
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++) dmma(acc[1][cb], a1, bv[cb]);
-    } else {
-      const double *b1 = B1 + (size_t)(k0 + kr) * ldb + rc;
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++) bv[cb] = GLOBAL_B ? __ldg(b1 + 8 * cb) : b1[8 * cb];
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++) dmma(acc[1][cb], a1, bv[cb]);
+    for (int q = 0; q < 4; q++) {
+      dmma(acc[2 * q], v[s], b[q].x);
+      dmma(acc[2 * q + 1], v[s], b[q].y);
     }
   }
+#pragma unroll
+  for (int s = 0; s < 16; s++) v[s] = acc[s >> 1][s & 1];
 }
 
-template <bool SAFE>
-__device__ __forceinline__ void child_v_mma(const DevCtx &c, const TileMap1 &tm, int kind, int id,
-                                            const double *et, const double *leaf, double *sA,
-                                            int w, int lane, double (&v)[2][8][2], int (&s)[2]) {
-  const int kr = lane & 3, rc = lane >> 2;
-  if (kind == GEMS_CHILD_TIP) {
-#pragma unroll
-    for (int rb = 0; rb < 2; rb++) {
-      const int r = 16 * w + 8 * rb + rc;
-      const bool ok = tm.valid(r);
-      const int st = ok ? min((int)c.tips[(size_t)id * c.P + tm.pattern(r)], c.unknown) : 0;
-      const double *row = leaf + ((size_t)st * tm.C + tm.cat(r)) * kN;
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int col = 8 * cb + 2 * kr + e;
-          v[rb][cb][e] = ok && col < kN ? __ldg(row + col) : 0.0;
-        }
-      s[rb] = 0;
-    }
-    return;
-  }
-  {
-    const char *e0 = reinterpret_cast<const char *>(et);
-    const int lines = (int)(et_doubles(tm.C) * sizeof(double) / 128);
-    for (int l = threadIdx.x; l < lines; l += blockDim.x)
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(e0 + (size_t)l * 128));
-  }
-  const double *src = static_cast<const double *>(c.partials) + (size_t)id * c.slot_elems;
-  constexpr int kPer = kRows * kK / kThreadsG;
-  static_assert(kRows * kK % kThreadsG == 0, "whole loads per thread");
-  double a[kPer];
-#pragma unroll
-  for (int u = 0; u < kPer; u++) {
-    const int idx = threadIdx.x + u * kThreadsG;
-    const int g = idx / kK, k = idx - g * kK;
-    a[u] = (tm.row_ok(g) && k < kN) ? __ldcg(src + tm.slot_row(g) * kN + k) : 0.0;
-  }
-#pragma unroll
-  for (int u = 0; u < kPer; u++) {
-    const int idx = threadIdx.x + u * kThreadsG;
-    const int g = idx / kK, k = idx - g * kK;
-    const int r = tm.tile_row(g);
-    if (r >= 0) sA[k * kLdM + r] = a[u];
-  }
-  const uint16_t *sc = c.scale + (size_t)id * c.slot_scale;
-#pragma unroll
-  for (int rb = 0; rb < 2; rb++) {
-    const int r = 16 * w + 8 * rb + rc;
-    const long p = tm.pattern(r);
-    s[rb] = tm.valid(r) ? (SAFE ? sc[(size_t)p * tm.C + tm.cat(r)] : sc[p]) : 0;
-  }
+// Op tables of the SAFE form, grid (nops, 2 sides, C): per side and category, an internal child's
+// E_c in fragment order, or a tip child's messages [state code][8][4 lanes][2] (E_c . tip vector,
+// 1 for the unknown state) in the order its rows are read.
+constexpr int kTipRow = 64;  // doubles per state code
+__global__ void __launch_bounds__(256) k_prep_ops_g61w(DevCtx c, const DevOp *ops, double *tab,
+                                                       size_t stride) {
+  extern __shared__ __align__(16) double sE[];  // [kFrag]
+  __shared__ double d[kK];
+  const int k = blockIdx.x, side = blockIdx.y, cc = blockIdx.z;
+  const DevOp op = ops[k];
+  const double len = side ? op.r_len : op.l_len;
+  for (int i = threadIdx.x; i < kN; i += blockDim.x) d[i] = exp(c.eval[i] * (c.rates[cc] * len));
   __syncthreads();
-  const double *b = et + (size_t)tm.c0 * kK * kNC;
-  gemm_mma<true>(sA, b, b, kNC, w, lane, v);
+  double *out = tab + (size_t)k * stride + ((size_t)side * c.C + cc) * kFrag;
+  const bool tip = (side ? op.r_kind : op.l_kind) == GEMS_CHILD_TIP;
+  for (int i = threadIdx.x; i < kFrag; i += blockDim.x) {
+    int kk, x;
+    frag_place(i, kk, x);
+    const double v = kk < kN && x < kN ? c.evec[x * kN + kk] * d[kk] : 0.0;
+    if (tip)
+      sE[i] = v;
+    else
+      out[i] = v;
+  }
+  if (!tip) return;
+  __syncthreads();
+  // a warp's 8 state codes: rows of tip vectors times E_c, summed in index order
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int st = 8 * (threadIdx.x >> 5) + g;
+  double v[16];
+#pragma unroll
+  for (int s = 0; s < 16; s++)
+    v[s] = st < c.unknown && 4 * s + t < kN ? c.tip[(size_t)st * kN + 4 * s + t] : 0.0;
+  product(sE, lane, v);
+  if (st > c.unknown) return;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const double a = st == c.unknown ? 1.0 : v[2 * q], b = st == c.unknown ? 1.0 : v[2 * q + 1];
+    reinterpret_cast<double2 *>(out + st * kTipRow)[q * 4 + t] = make_double2(a, b);
+  }
 }
 
-template <bool SAFE>
-__global__ void __launch_bounds__(kThreadsG, 2)
-    k_traverse_g61m(DevCtx c, const DevOp *__restrict__ ops, int nops,
+__global__ void __launch_bounds__(kThreadsW, 2)
+    k_traverse_g61w(DevCtx c, const DevOp *__restrict__ ops, int nops,
                     const double *__restrict__ tab, size_t stride, int tile0) {
-  static_assert(SAFE, "one category per tile: SAFE scaling only");
   extern __shared__ __align__(16) double smem[];
-  double *sIv = smem;                  // [kK][kLdM]: inv_evec[j][x] at [x][j]
-  double *sA = sIv + kK * kLdM;        // [kK][kLdM]
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, kr = lane & 3, rc = lane >> 2;
-  TileMap1 tm;
-  tm.C = c.C;
-  tm.tp = kRows;
-  tm.nrow = kRows;
-  tm.c0 = blockIdx.x % c.C;
-  tm.p0 = (long)(tile0 + blockIdx.x / c.C) * kRows;
-  tm.P = c.P;
-  for (int idx = threadIdx.x; idx < kK * kLdM; idx += blockDim.x) {
-    const int k = idx / kLdM, x = idx - k * kLdM;
-    sIv[idx] = (k < kN && x < kN) ? c.inv_evec[x * kN + k] : 0.0;
-    sA[idx] = 0.0;  // rows past the tile's rows (64 % C) are never written
+  double *sInv = smem, *sE = smem + kFrag;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int cat = blockIdx.x % c.C;
+  const long p = (long)(tile0 + blockIdx.x / c.C) * kRows + 8 * (tid >> 5) + g;
+  const bool act = p < c.P;
+  const size_t row = ((size_t)p * c.C + cat) * kN;
+  for (int i = tid; i < kFrag; i += kThreadsW) {
+    int kk, x;
+    frag_place(i, kk, x);
+    sInv[i] = kk < kN && x < kN ? c.inv_evec[x * kN + kk] : 0.0;
   }
   double *part = static_cast<double *>(c.partials);
-  const int blk = c.C * kN;
-  for (int kop = 0; kop < nops; kop++) {
-    const DevOp op = ops[kop];
-    const double *tk = tab + (size_t)kop * stride;
-    const double *leafL = tk + 2 * et_doubles(c.C);
-    const double *leafR = leafL + (size_t)(c.unknown + 1) * blk;
+  const bool inv0 = act && c.invar[p] == 0.0;
+
+  // the side of an op that is worked on first: the forwarded child, which is in registers
+  auto first_side = [](const DevOp &o) {
+    return o.r_kind == GEMS_CHILD_PARTIAL && plan_rsrc(o.pad_) == kSrcFwd ? 1 : 0;
+  };
+  // the next internal child in working order from (op k, position i), and its E_c into a slot
+  int nk = 0, ni = 0, nslot = 0;
+  auto fetch_next = [&]() {
+    for (; nk < nops; nk++, ni = 0) {
+      const DevOp o = ops[nk];
+      for (; ni < 2; ni++) {
+        const int side = ni ^ first_side(o);
+        if ((side ? o.r_kind : o.l_kind) != GEMS_CHILD_PARTIAL) continue;
+        const double *src =
+            tab + (size_t)nk * stride + ((size_t)side * c.C + cat) * kFrag + 2 * tid;
+        const uint32_t dst = static_cast<uint32_t>(
+            __cvta_generic_to_shared(sE + (size_t)(nslot & 1) * kFrag + 2 * tid));
+#pragma unroll
+        for (int j = 0; j < kFrag / 2 / kThreadsW; j++)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                           dst + j * kThreadsW * 16),
+                       "l"(src + j * kThreadsW * 2)
+                       : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        nslot++;
+        ni++;
+        return;
+      }
+    }
+  };
+  fetch_next();
+  int slot = 0;
+  // message of an internal child: its E_c has come for every warp, and every warp is done with
+  // the slot before it, which the next one's copy may fill
+  auto message = [&](double (&v)[16]) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    fetch_next();
+    product(sE + (size_t)(slot & 1) * kFrag, lane, v);
+    slot++;
+  };
+
+  __syncthreads();  // sInv, before any warp's first product
+  double x[16];
+  int sx = 0;  // counter of x
+#pragma unroll
+  for (int s = 0; s < 16; s++) x[s] = 0.0;
+  for (int k = 0; k < nops; k++) {
+    const DevOp op = ops[k];
+    const double *tk = tab + (size_t)k * stride;
+    const int first = first_side(op);
+    const bool fwd = first || (op.l_kind == GEMS_CHILD_PARTIAL && plan_lsrc(op.pad_) == kSrcFwd);
     const bool tiptip = op.l_kind == GEMS_CHILD_TIP && op.r_kind == GEMS_CHILD_TIP;
-    double vl[2][8][2], o[2][8][2];
-    int sl[2], sr[2];
-    __syncthreads();
-    child_v_mma<SAFE>(c, tm, op.l_kind, op.l_id, tk, leafL, sA, w, lane, vl, sl);
-    __syncthreads();
-    child_v_mma<SAFE>(c, tm, op.r_kind, op.r_id, tk + et_doubles(c.C), leafR, sA, w, lane, o, sr);
-    __syncthreads();
+    // a child's elements and counter
+    auto load = [&](int side, double (&v)[16], int &s) {
+      const int kind = side ? op.r_kind : op.l_kind, id = side ? op.r_id : op.l_id;
+      s = 0;
 #pragma unroll
-    for (int rb = 0; rb < 2; rb++)
+      for (int q = 0; q < 16; q++) v[q] = 0.0;
+      if (!act) return;
+      if (kind == GEMS_CHILD_TIP) {
+        const int st = min((int)c.tips[(size_t)id * c.P + p], c.unknown);
+        const double2 *q = reinterpret_cast<const double2 *>(
+                               tk + ((size_t)side * c.C + cat) * kFrag + st * kTipRow) + t;
 #pragma unroll
-      for (int cb = 0; cb < 8; cb++)
-#pragma unroll
-        for (int e = 0; e < 2; e++)
-          sA[(8 * cb + 2 * kr + e) * kLdM + 16 * w + 8 * rb + rc] = vl[rb][cb][e] * o[rb][cb][e];
-    __syncthreads();
-    gemm_mma<false>(sA, sIv, sIv, kLdM, w, lane, o);
-    double m[2];
-#pragma unroll
-    for (int rb = 0; rb < 2; rb++) {
-      double x = 0.0;
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++) x = fmax(x, fmax(fabs(o[rb][cb][0]), fabs(o[rb][cb][1])));
-      x = fmax(x, __shfl_xor_sync(0xffffffffu, x, 1));
-      x = fmax(x, __shfl_xor_sync(0xffffffffu, x, 2));
-      m[rb] = x;
-    }
-    uint16_t *scd = c.scale + (size_t)op.dst_slot * c.slot_scale;
-    double *dst = part + (size_t)op.dst_slot * c.slot_elems;
-#pragma unroll
-    for (int rb = 0; rb < 2; rb++) {
-      const int r = 16 * w + 8 * rb + rc;
-      if (!tm.valid(r)) continue;
-      const long p = tm.pattern(r);
-      const int cat = tm.cat(r);
-      int s_out = sl[rb] + sr[rb];
-      const bool scale = !tiptip && m[rb] < kScaleThr && c.invar[p] == 0.0;
-      if (scale) s_out += 1;
-      double *row = dst + tm.off(r);
-#pragma unroll
-      for (int cb = 0; cb < 8; cb++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int col = 8 * cb + 2 * kr + e;
-          if (col < kN) row[col] = scale ? ldexp(o[rb][cb][e], kScaleExp) : o[rb][cb][e];
+        for (int j = 0; j < 8; j++) {
+          const double2 a = __ldg(q + 4 * j);
+          v[2 * j] = a.x, v[2 * j + 1] = a.y;
         }
-      if (kr == 0) scd[(size_t)p * tm.C + cat] = (uint16_t)s_out;
+      } else {
+        const double *q = part + (size_t)id * c.slot_elems + row + t;
+#pragma unroll
+        for (int j = 0; j < 15; j++) v[j] = __ldcg(q + 4 * j);
+        if (t == 0) v[15] = __ldcg(q + 60);
+        s = c.scale[(size_t)id * c.slot_scale + (size_t)p * c.C + cat];
+      }
+    };
+    double y[16];
+    int sy;
+    if (!fwd) load(first, x, sx);
+    if ((first ? op.r_kind : op.l_kind) == GEMS_CHILD_PARTIAL) message(x);
+    load(1 - first, y, sy);
+    if ((first ? op.l_kind : op.r_kind) == GEMS_CHILD_PARTIAL) message(y);
+#pragma unroll
+    for (int s = 0; s < 16; s++) x[s] *= y[s];
+    product(sInv, lane, x);
+    // |x| by its high word, NaN as 0: a maximum that ignores NaN, compared with a power of two
+    int h = 0;
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+      const int w = __double2hiint(x[s]) & 0x7fffffff;
+      h = max(h, w > 0x7ff00000 ? 0 : w);
     }
+    h = max(h, __shfl_xor_sync(0xffffffffu, h, 1));
+    h = max(h, __shfl_xor_sync(0xffffffffu, h, 2));
+    sx += sy;
+    if (!tiptip && h < 0x2FF00000 /* 2^-256 */ && inv0) {
+#pragma unroll
+      for (int s = 0; s < 16; s++) x[s] *= 0x1p256;
+      sx += 1;
+    }
+    if (act) {
+      double *q = part + (size_t)op.dst_slot * c.slot_elems + row + t;
+#pragma unroll
+      for (int j = 0; j < 15; j++) q[4 * j] = x[j];
+      if (t == 0) {
+        q[60] = x[15];
+        c.scale[(size_t)op.dst_slot * c.slot_scale + (size_t)p * c.C + cat] = (uint16_t)sx;
+      }
+    }
+    __syncwarp();  // the counter that lane t = 0 wrote is read by its pattern's four lanes
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 }  // namespace
@@ -511,8 +535,12 @@ bool g61_supported(const Session *s) {
 
 int launch_prep_ops_g61(Session *s, int nops) {
   if (nops <= 0) return GEMS_OK;
-  k_prep_ops_g61<<<dim3(nops, 2), 256, 0, s->stream>>>(s->ctx(), s->d_ops, s->d_opmats,
-                                                        s->op_stride);
+  if (s->desc.scaling == GEMS_SCALE_SAFE)
+    k_prep_ops_g61w<<<dim3(nops, 2, s->desc.ncat), 256, sizeof(double) * kFrag, s->stream>>>(
+        s->ctx(), s->d_ops, s->d_opmats, s->op_stride);
+  else
+    k_prep_ops_g61<<<dim3(nops, 2), 256, 0, s->stream>>>(s->ctx(), s->d_ops, s->d_opmats,
+                                                          s->op_stride);
   s->launches++;
   GEMS_CUDA(cudaGetLastError());
   return GEMS_OK;
@@ -539,11 +567,10 @@ int launch_traverse_g61(Session *s, int nops, int p0, int p1) {
   // value
   if (safe) {  // FP64 tensor cores, one category per tile
     const int g = ((p1 + kRows - 1) / kRows - tile0) * s->desc.ncat;
-    GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61m<true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemM));
-    k_traverse_g61m<true><<<g, kThreadsG, kSmemM, s->stream>>>(s->ctx(), s->d_ops, nops,
-                                                                s->d_opmats, s->op_stride,
-                                                                tile0);
+    GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61w, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kSmemW));
+    k_traverse_g61w<<<g, kThreadsW, kSmemW, s->stream>>>(s->ctx(), s->d_ops, nops, s->d_opmats,
+                                                         s->op_stride, tile0);
   } else {  // NORM: a pattern's categories in one tile, FP64 FMA
     GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61<false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemG));
