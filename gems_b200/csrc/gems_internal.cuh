@@ -178,9 +178,7 @@ struct Session {
   double *d_model = nullptr;  // eval | evec | inv_evec | rates | props | tip | tip_real
   DevOp *d_ops = nullptr;
   double *d_opmats = nullptr;
-  double *d_branch = nullptr;  // per-branch tables: val0,val1,val2 [block] + tip table
   double *d_red = nullptr;     // reduction partials
-  double *d_result = nullptr;  // final scalars
   int *d_flag = nullptr;       // device status flags (barrier timeouts)
   unsigned int *d_bar = nullptr;  // count of finished blocks of a branch-term launch (zero between)
   void *d_slots = nullptr;        // the Newton kernel's exchange slots

@@ -25,7 +25,7 @@
 // Measured on one 200-taxon codon model (3,780 patterns, +G4), a from-scratch traversal: per-row
 // kernel 26.6 ms; FMA tiles of 128 rows 7.0 ms, with the L1 prefetch 5.9 ms, 64-row tiles at two
 // CTAs per SM 5.3 ms; mma over rows staged in shared memory between products 4.7 ms; chained in
-// registers 2.4 ms.  lnL and eight branch derivatives of that model: 11.6 -> 5.0 ms with the last
+// registers 2.05 ms.  lnL and eight branch derivatives of that model: 11.6 -> 5.0 ms with the last
 // form, its op tables (mma as well, 17 us where one thread per element took 234) included.
 #include <string>
 

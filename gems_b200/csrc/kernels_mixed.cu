@@ -9,7 +9,8 @@
 // counter is incremented; each count is worth 64*log(2) in the log-likelihood.
 // The branch terms are FP64: both partials are lifted to the eigen basis in FP64
 // (inv_evec . real), and theta / the log-likelihood reduction / the derivative sums / Newton
-// reuse the FP64 kernels, so every accepted length is re-evaluated in FP64.
+// are the FP64 kernels' (kernels_branch.cu), so every accepted length is re-evaluated in FP64.
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <string>
@@ -26,15 +27,6 @@ __device__ __forceinline__ float group_maxf(float v, int G) {
   for (int o = 1; o < G; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ double group_sum(double v, int G) {
-  for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ int group_min(int v, int G) {
-  for (int o = 1; o < G; o <<= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 template <int K>
 __device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[32]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -214,124 +206,146 @@ __global__ void __launch_bounds__(kThreads) k_traverse_mixed(DevCtx c, const Dev
   }
 }
 
-// eigen-basis FP64 lift of one category of a real FP32 partial (or of a tip indicator)
-template <int N>
-__device__ __forceinline__ void lift(const DevCtx &c, const float (&a)[N], double (&e)[N]) {
-#pragma unroll 4
-  for (int i = 0; i < N; i++) {
-    double acc = 0.0;
-#pragma unroll
-    for (int x = 0; x < N; x++) acc = fma(__ldg(c.inv_evec + i * N + x), (double)a[x], acc);
-    e[i] = acc;
-  }
+// ----------------------------------------------------------------------------------------
+// theta (FP64, eigen basis) of a 20- or 61-state branch from its FP32 real partials, and its lnL.
+// Lifting a row to the eigen basis is a product with inv_evec, done on the FP64 mma (m8n8k4) for
+// the 8 patterns of a warp, both ends of the branch on the same fragments of inv_evec.  Lane
+// (g, t) = (lane / 4, lane % 4) holds the states 4s + t of pattern g as A fragments (K steps s) and,
+// with column n = 2 t' + e of N tile m standing for state 8m + 4e + t', the same states of the
+// result; a warp reads 128 contiguous bytes of the tile-major partials per K step, and the sums
+// run in index order.
+// Bound by FP64 throughput, 2 x 8 x 16 mma a category and 8 patterns for 61 states: 23 us for
+// 3,780 patterns of 61 states and 50 us for 98,762 of 20 (4 categories), where one thread per
+// (pattern, category) with its rows in local memory took 65 and 74.  The last block adds the
+// blocks' sums in index order and writes them to pinned host memory.
+// ----------------------------------------------------------------------------------------
+constexpr int kWarpsL = 4;
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 
-// theta (FP64, eigen basis) from FP32 real partials; also the branch lnL when want_lnl.
 template <int N, bool SAFE>
-__global__ void __launch_bounds__(kThreads) k_theta_mixed(DevCtx c, gems_branch br, int want_lnl,
-                                                          int store_theta,
-                                                          const double *__restrict__ val) {
+__global__ void __launch_bounds__(32 * kWarpsL, N == 61 ? 3 : 5)
+    k_theta_mixed(DevCtx c, gems_branch br, int want_lnl, int store_theta, unsigned int *ticket,
+                  double *out) {
+  constexpr int S = (N + 3) / 4, M = (N + 7) / 8;
+  static_assert(mix_k<N>() == S, "K steps are the chunks of the tile-major rows");
+  extern __shared__ double sm[];  // inv_evec as B fragments [S][M][32], then val [C][N]
   __shared__ double sh[2][32];
-  const int G = c.G;
-  const int gl = threadIdx.x & (G - 1);
-  const long p = ((long)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const bool act = p < c.P && gl < c.C;
-  const float *part = static_cast<const float *>(c.partials);
-  int ssum = 0;
-  double th[N];
-  if (act) {
-    float a[N];
-    load_vecf<N>(part + (size_t)br.dad_slot * c.slot_elems + mix_off<N>(c, p, gl), a, mix_cs<N>());
-    double de[N];
-    lift<N>(c, a, de);
-    const uint16_t *sd = c.scale + (size_t)br.dad_slot * c.slot_scale;
-    ssum = SAFE ? sd[(size_t)p * c.C + gl] : sd[p];
-    if (br.node_kind == GEMS_CHILD_TIP) {
-      const int st = c.tips[(size_t)br.node_id * c.P + p];
-      const double *tp = c.tip + (size_t)st * N;
-#pragma unroll
-      for (int i = 0; i < N; i++) th[i] = __ldg(tp + i) * de[i];
-    } else {
-      float b[N];
-      load_vecf<N>(part + (size_t)br.node_id * c.slot_elems + mix_off<N>(c, p, gl), b, mix_cs<N>());
-      double ne[N];
-      lift<N>(c, b, ne);
-#pragma unroll
-      for (int i = 0; i < N; i++) th[i] = ne[i] * de[i];
-      const uint16_t *sn = c.scale + (size_t)br.node_id * c.slot_scale;
-      ssum += SAFE ? sn[(size_t)p * c.C + gl] : sn[p];
-    }
+  __shared__ bool last;
+  double *val = sm + S * M * 32;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int i = threadIdx.x; i < S * M * 32; i += blockDim.x) {
+    const int l = i & 31, m = (i >> 5) % M, k = 4 * ((i >> 5) / M) + (l & 3), n = l >> 2;
+    const int x = 8 * m + 4 * (n & 1) + (n >> 1);
+    sm[i] = k < N && x < N ? c.inv_evec[x * N + k] : 0.0;
   }
-  int ms = ssum;
-  if (SAFE) {
-    ms = group_min(act ? ssum : INT_MAX, G);
-    if (act) {
+  if (want_lnl)
+    for (int i = threadIdx.x; i < c.block; i += blockDim.x)
+      val[i] = exp(c.eval[i % N] * (c.rates[i / N] * br.length)) * c.props[i / N];
+  __syncthreads();
+  const float *part = static_cast<const float *>(c.partials);
+  const float *dad = part + (size_t)br.dad_slot * c.slot_elems;
+  const float *node = part + (size_t)br.node_id * c.slot_elems;
+  const uint16_t *sd = c.scale + (size_t)br.dad_slot * c.slot_scale;
+  const uint16_t *sn = c.scale + (size_t)br.node_id * c.slot_scale;
+  const bool is_tip = br.node_kind == GEMS_CHILD_TIP;
+  double v[2] = {0.0, 0.0};
+  // P is a multiple of 64: whole warps of patterns
+  for (long p0 = 8l * ((long)blockIdx.x * kWarpsL + (threadIdx.x >> 5)); p0 < c.P;
+       p0 += 8l * kWarpsL * gridDim.x) {
+    const long p = p0 + g;
+    const int st = is_tip ? min((int)c.tips[(size_t)br.node_id * c.P + p], c.unknown) : 0;
+    int ms;
+    if (SAFE) {
+      ms = INT_MAX;
+      for (int cc = t; cc < c.C; cc += 4)
+        ms = min(ms, (int)sd[p * c.C + cc] + (is_tip ? 0 : (int)sn[p * c.C + cc]));
+      ms = min(ms, __shfl_xor_sync(0xffffffffu, ms, 1));
+      ms = min(ms, __shfl_xor_sync(0xffffffffu, ms, 2));
+    } else {
+      ms = (int)sd[p] + (is_tip ? 0 : (int)sn[p]);
+    }
+    double lh = 0.0;
+    for (int cc = 0; cc < c.C; cc++) {
+      const size_t o = mix_off<N>(c, p, cc) + t;
+      float a[S], b[S];
+#pragma unroll
+      for (int s = 0; s < S; s++) {
+        a[s] = __ldcg(dad + o + (size_t)s * mix_cs<N>());
+        b[s] = is_tip ? 0.f : __ldcg(node + o + (size_t)s * mix_cs<N>());
+      }
+      int ss = ms;
+      if (SAFE) ss = (int)sd[p * c.C + cc] + (is_tip ? 0 : (int)sn[p * c.C + cc]);
+      double x[M][2], y[M][2];
+#pragma unroll
+      for (int m = 0; m < M; m++) x[m][0] = x[m][1] = y[m][0] = y[m][1] = 0.0;
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < S; s++) {
+        double f[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) f[m] = sm[(s * M + m) * 32 + lane];
+#pragma unroll
+        for (int m = 0; m < M; m++) dmma(x[m], (double)a[s], f[m]);
+        if (!is_tip) {
+#pragma unroll
+          for (int m = 0; m < M; m++) dmma(y[m], (double)b[s], f[m]);
+        }
+      }
       // a category one count above the minimum is 2^-64 smaller; two or more: negligible
-      if (ssum == ms + 1) {
+      const double up = ss == ms ? 1.0 : 5.421010862427522e-20;
+      double *dst = c.theta + (size_t)p * c.block + cc * N + t;
 #pragma unroll
-        for (int i = 0; i < N; i++) th[i] *= 5.421010862427522e-20;  // 2^-64
-      } else if (ssum > ms + 1) {
-#pragma unroll
-        for (int i = 0; i < N; i++) th[i] = 0.0;
+      for (int s = 0; s < S; s++) {
+        if (4 * s + t >= N) continue;
+        const double e =
+            is_tip ? __ldg(c.tip + (size_t)st * N + 4 * s + t) : y[s >> 1][s & 1];
+        double th = e * x[s >> 1][s & 1];
+        if (SAFE) th = ss > ms + 1 ? 0.0 : th * up;
+        if (store_theta) dst[4 * s] = th;
+        if (want_lnl) lh = fma(val[cc * N + 4 * s + t], th, lh);
+      }
+    }
+    if (store_theta && t == 0) c.scale_all[p] = (double)ms * kLogScaleThrF;
+    if (!want_lnl) continue;
+    lh += __shfl_xor_sync(0xffffffffu, lh, 1);
+    lh += __shfl_xor_sync(0xffffffffu, lh, 2);
+    if (t == 0) {
+      const double plh = log(fabs(lh) + c.invar[p]) + ms * kLogScaleThrF;
+      c.pattern_lh[p] = plh;
+      if (p < c.nptn) {
+        const double f = c.freq[p];
+        v[0] += plh * f;
+        v[1] += (isfinite(plh) ? plh : 4.0 * kLogScaleThr) * f;
       }
     }
   }
-  if (act && store_theta) {
-    double *dst = c.theta + (size_t)p * c.block + gl * N;
-#pragma unroll
-    for (int i = 0; i < N; i++) dst[i] = th[i];
-    if (gl == 0) c.scale_all[p] = (double)ms * kLogScaleThrF;
-  }
   if (!want_lnl) return;
-  double lh_cat = 0.0;
-  if (act) {
-#pragma unroll
-    for (int i = 0; i < N; i++) lh_cat = fma(__ldg(val + gl * N + i), th[i], lh_cat);
+  block_sum<2>(v, sh);
+  if (threadIdx.x == 0) {
+    __stcg(c.red + 2 * blockIdx.x, v[0]);
+    __stcg(c.red + 2 * blockIdx.x + 1, v[1]);
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
-  const double lh_sum = group_sum(lh_cat, G);
-  double v[2] = {0.0, 0.0};
-  if (act && gl == 0) {
-    const double lh = fabs(lh_sum) + c.invar[p];
-    const double plh = log(lh) + ms * kLogScaleThrF;
-    c.pattern_lh[p] = plh;
-    if (p < c.nptn) {
-      const double f = c.freq[p];
-      v[0] = plh * f;
-      v[1] = (isfinite(plh) ? plh : 4.0 * kLogScaleThr) * f;
-    }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v[0] = v[1] = 0.0;
+  for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+    v[0] += __ldcg(c.red + 2 * b);
+    v[1] += __ldcg(c.red + 2 * b + 1);
   }
   block_sum<2>(v, sh);
   if (threadIdx.x == 0) {
-    c.red[2 * blockIdx.x] = v[0];
-    c.red[2 * blockIdx.x + 1] = v[1];
+    out[0] = v[0];
+    out[1] = v[1];
+    *ticket = 0;  // ready for the next launch
   }
-}
-
-__global__ void k_val_table(DevCtx c, double len, double *val) {
-  for (int idx = threadIdx.x; idx < c.block; idx += blockDim.x) {
-    const int cc = idx / c.n, i = idx - cc * c.n;
-    val[idx] = exp(c.eval[i] * (c.rates[cc] * len)) * c.props[cc];
-  }
-}
-
-template <int K>
-__global__ void k_reduce_final_m(const double *red, int nblk, double *out) {
-  __shared__ double sh[K][32];
-  double v[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) v[k] = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] += red[(size_t)K * b + k];
-  block_sum<K>(v, sh);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < K; k++) out[k] = v[k];
-}
-
-inline int grid_for(const Session *s) {
-  const long threads = (long)s->P * s->G;
-  return (int)((threads + kThreads - 1) / kThreads);
 }
 
 }  // namespace
@@ -375,29 +389,20 @@ int launch_traverse_mixed(Session *s, int nops, int p0, int p1) {
 // theta (and optionally the branch lnL) from the two FP32 partials of br, 20 or 61 states
 int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta) {
   DevCtx c = s->ctx();
-  const int grid = grid_for(s);
+  const int n = s->desc.nstates;
   const bool safe = s->desc.scaling == GEMS_SCALE_SAFE;
-  double *val = s->d_branch;
-  if (want_lnl) {
-    k_val_table<<<1, 256, 0, s->stream>>>(c, br->length, val);
-    s->launches++;
-  }
+  const size_t smem =
+      sizeof(double) * ((size_t)((n + 3) / 4) * ((n + 7) / 8) * 32 + (want_lnl ? s->block : 0));
+  const int grid = std::min(148 * (n == 61 ? 3 : 5), (s->P / 8 + kWarpsL - 1) / kWarpsL);
   cudaEvent_t ev0;
   if (int st = prof_begin(s, want_lnl ? 1 : 2, &ev0)) return st;
   const int wl = want_lnl ? 1 : 0, stt = store_theta ? 1 : 0;
-  auto *fn = s->desc.nstates == 20 ? (safe ? k_theta_mixed<20, true> : k_theta_mixed<20, false>)
-                                   : (safe ? k_theta_mixed<61, true> : k_theta_mixed<61, false>);
-  fn<<<grid, kThreads, 0, s->stream>>>(c, *br, wl, stt, val);
+  auto *fn = n == 20 ? (safe ? k_theta_mixed<20, true> : k_theta_mixed<20, false>)
+                     : (safe ? k_theta_mixed<61, true> : k_theta_mixed<61, false>);
+  fn<<<grid, 32 * kWarpsL, smem, s->stream>>>(c, *br, wl, stt, s->d_bar, s->h_result);
   s->launches++;
   GEMS_CUDA(cudaGetLastError());
-  if (int st = prof_end(s, want_lnl ? 1 : 2, ev0)) return st;
-  if (!want_lnl) return GEMS_OK;
-  k_reduce_final_m<2><<<1, 256, 0, s->stream>>>(s->d_red, grid, s->d_result);
-  s->launches++;
-  GEMS_CUDA(cudaGetLastError());
-  GEMS_CUDA(cudaMemcpyAsync(s->h_result, s->d_result, 2 * sizeof(double), cudaMemcpyDeviceToHost,
-                            s->stream));
-  return GEMS_OK;
+  return prof_end(s, want_lnl ? 1 : 2, ev0);
 }
 
 }  // namespace gems

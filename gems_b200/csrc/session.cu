@@ -188,12 +188,9 @@ static void free_session(Session *s) {
   cudaFree(s->d_model);
   cudaFree(s->d_ops);
   cudaFree(s->d_opmats);
-  cudaFree(s->d_branch);
   cudaFree(s->d_red);
-  cudaFree(s->d_result);
   cudaFree(s->d_flag);
   cudaFree(s->d_bar);
-  cudaFree(s->d_slots);
   cudaFreeHost(s->h_ops);
   cudaFree(s->d_jobs);
   cudaFreeHost(s->h_jobs);
@@ -495,12 +492,10 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
   ALLOC(s->d_model, z.model_doubles * sizeof(double));
   ALLOC(s->d_ops, (size_t)z.nops_max * sizeof(DevOp));
   ALLOC(s->d_opmats, z.opmats_bytes);
-  ALLOC(s->d_branch, z.branch_bytes);
   ALLOC(s->d_red, z.red_doubles * sizeof(double));
-  ALLOC(s->d_result, 16 * sizeof(double));
   ALLOC(s->d_flag, 16 * sizeof(int));
-  ALLOC(s->d_bar, 16 * sizeof(unsigned int));
-  ALLOC(s->d_slots, newton_slot_bytes());
+  ALLOC(s->d_bar, 128 + newton_slot_bytes());  // then the Newton exchange's slots
+  s->d_slots = reinterpret_cast<char *>(s->d_bar) + 128;
 #undef ALLOC
   if ((e = cudaHostAlloc((void **)&s->h_ops, (size_t)z.nops_max * sizeof(DevOp), 0)) !=
       cudaSuccess)
@@ -519,8 +514,7 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
       (e = cudaMemsetAsync(s->d_freq, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_invar, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_scale, 0, z.scale_bytes, s->stream)) ||
-      (e = cudaMemsetAsync(s->d_bar, 0, 16 * sizeof(unsigned int), s->stream)) ||
-      (e = cudaMemsetAsync(s->d_slots, 0, newton_slot_bytes(), s->stream)) ||
+      (e = cudaMemsetAsync(s->d_bar, 0, 128 + newton_slot_bytes(), s->stream)) ||
       (e = cudaStreamSynchronize(s->stream)))
     return fail(e, "initialise session");
   *out = s;
