@@ -796,7 +796,7 @@ double terms_lnl(const Session *s) {
 
 int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf) {
   if (int st = enqueue_terms(s, br, br != nullptr, false, length)) return st;
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  if (int st = sync_session(s)) return st;
   *df = s->h_result[0];
   *ddf = s->h_result[1];
   if (!std::isfinite(*df)) *df = *ddf = 0.0;  // phylokernelnew.h:2646-2649
@@ -805,7 +805,7 @@ int launch_derv(Session *s, const gems_branch *br, double length, double *df, do
 
 int launch_from_buffer(Session *s, double length, double *lnl) {
   if (int st = enqueue_terms(s, nullptr, false, true, length)) return st;
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  if (int st = sync_session(s)) return st;
   *lnl = terms_lnl(s);
   return GEMS_OK;
 }
@@ -813,7 +813,7 @@ int launch_from_buffer(Session *s, double length, double *lnl) {
 size_t newton_slot_bytes() { return sizeof(ulonglong2) * 2 * kMaxClusters * kSlotStride; }
 
 int newton_result(Session *s, double *opt_len, int *nevals) {
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  if (int st = sync_session(s)) return st;
   *opt_len = s->h_result[0];
   *nevals = (int)s->h_result[1];
   return (int)s->h_result[2];
