@@ -257,17 +257,23 @@ int launch_traverse(Session *s, int nops, int p0, int p1);
 // branch terms (kernels_branch.cu).  theta_in_kernel: theta is formed by the kernel that uses it
 // (else launch it first: enqueue_theta_mixed); br null: theta as stored
 bool theta_in_kernel(const Session *s);
+// whether a branch call runs these node updates in its own launch (`ops` of the calls below;
+// validated by the caller)
+bool small_ops(const Session *s, int nops);
 // lnL or derivatives at `length`, theta kept with `store`; the results are in s->h_result once
 // the session's stream has completed (terms_lnl: the lnL of them)
-int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length);
+int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length,
+                  const gems_op *ops, int nops);
 double terms_lnl(const Session *s);
-int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf);
+int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf,
+                const gems_op *ops, int nops);
 int launch_from_buffer(Session *s, double length, double *lnl);
 // the Newton loop in two halves: enqueue (result written to pinned host memory), then wait and
 // read
 size_t newton_slot_bytes();
 int launch_newton_async(Session *s, const gems_branch *br, double guess, double min_len,
-                        double max_len, double xacc, int max_steps);
+                        double max_len, double xacc, int max_steps, const gems_op *ops,
+                        int nops);
 int newton_result(Session *s, double *opt_len, int *nevals);
 int launch_eigen(Session *s, const double *exch_upper, const double *freq);
 // the same for nsess sessions of one state count in one launch (inputs stacked per session)

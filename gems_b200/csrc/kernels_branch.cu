@@ -20,7 +20,9 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "gems_internal.cuh"
 #include "tc_common.cuh"
@@ -38,6 +40,8 @@ enum : int {
   kM4        // FP32 real-space partials, 4 states: lifted to the eigen basis in FP64
 };
 enum : int { kStore = 1, kLnl = 2, kDerv = 4 };
+constexpr int kSmallOps = 16;           // ops of a list that a branch call runs itself
+constexpr int kSmallPatterns = 1 << 15;
 
 template <int SRC>
 __host__ __device__ constexpr int src_states() {
@@ -298,6 +302,206 @@ __device__ __forceinline__ void block_pair(double &a, double &b, double (*sh)[2]
   }
 }
 
+// ---- short op lists of 4-state sessions ---------------------------------------------------
+// A branch call that needs a few node updates first (the partials between the last branch and
+// this one) runs them in its own launch: with two pairs per lane (2 or more categories) a lane
+// holds one category's row of a pattern, which is all that a node update needs beside the
+// pattern's maximum.  The op list travels as a kernel parameter, the exponentials (mixed: P_c) are
+// made in shared memory by each block, the row that the last op wrote is kept, and everything is
+// stored as the traversal kernels store it: the same sums in the same order, the same bits.
+// This takes an op-list copy, a table launch and a traversal launch off the chain of a call: per
+// optimised branch of a 50-taxon tree with 18,501 patterns (FP64) 39 us -> 32, of NNI evaluations
+// of 4,703 (mixed) 49 -> 43, per branch derivative of 3,801 (FP64) 31 -> 23.
+struct SmallOps {
+  int n;
+  int pad;
+  DevOp op[kSmallOps];
+};
+template <int SRC, int E2>
+__host__ __device__ constexpr bool small_form() {
+  return (SRC == kT4 || SRC == kM4) && E2 == 2;
+}
+// doubles of dynamic shared memory: evec, inv_evec, exponentials [op][side][C][4], mixed: P_c
+// [op][side][C][16] floats
+__host__ __device__ inline int small_doubles(int n, int C, bool mixed) {
+  return n ? 32 + n * 2 * C * (mixed ? 12 : 4) : 0;
+}
+
+// by all threads of the block, followed by a barrier
+template <int SRC>
+__device__ __forceinline__ void small_tables(const DevCtx &c, const SmallOps &o, double *sm) {
+  const int C = c.C, n = o.n * 2 * C * 4;
+  double *ex = sm + 32;
+  for (int i = threadIdx.x; i < 32; i += blockDim.x) sm[i] = i < 16 ? c.evec[i] : c.inv_evec[i - 16];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int j = i & 3, cc = (i >> 2) % C, ks = (i >> 2) / C;
+    const DevOp &op = o.op[ks >> 1];
+    ex[i] = exp(c.eval[j] * (c.rates[cc] * (ks & 1 ? op.r_len : op.l_len)));
+  }
+  if constexpr (SRC == kM4) {
+    __syncthreads();
+    float *P = reinterpret_cast<float *>(ex + n);
+    for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) {
+      const int y = i & 3, x = (i >> 2) & 3;
+      const double *e = ex + (i >> 4) * 4;
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc = fma(sm[x * 4 + j] * e[j], sm[16 + j * 4 + y], acc);
+      P[i] = (float)fmax(acc, 0.0);
+    }
+  }
+}
+
+// the node updates of patterns p[0], p[1] (this lane: category l); all lanes of a warp call it
+template <int SRC, bool SAFE>
+__device__ __forceinline__ void small_traverse(const DevCtx &c, const SmallOps &o,
+                                               const double *sm, int L, int l,
+                                               const long (&p)[2]) {
+  using R = std::conditional_t<SRC == kM4, float, double>;
+  const int C = c.C, cat = l < C ? l : 0;
+  const bool act[2] = {p[0] < c.P && l < C, p[1] < c.P && l < C};
+  const bool inv0[2] = {act[0] && c.invar[p[0]] == 0.0, act[1] && c.invar[p[1]] == 0.0};
+  const double *ev = sm, *iv = sm + 16, *ex = sm + 32;
+  const float *Pm = reinterpret_cast<const float *>(ex + o.n * 2 * C * 4);
+  R *part = static_cast<R *>(c.partials);
+  R last[2][4];  // the row that the last op wrote, and its counter
+  int slast[2] = {0, 0}, slot = -1;
+#pragma unroll
+  for (int u = 0; u < 2; u++)
+#pragma unroll
+    for (int x = 0; x < 4; x++) last[u][x] = 0;
+  for (int k = 0; k < o.n; k++) {
+    const DevOp &op = o.op[k];
+    R v[2][2][4];  // [side][pattern][state]
+    int sc[2] = {0, 0};
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      const int kind = side ? op.r_kind : op.l_kind, id = side ? op.r_id : op.l_id;
+      const double *d = ex + ((2 * k + side) * C + cat) * 4;
+      const float4 *P = reinterpret_cast<const float4 *>(Pm) + ((2 * k + side) * C + cat) * 4;
+      R row[2][4];
+      if (kind == GEMS_CHILD_TIP) {
+        int st[2] = {0, 0};
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+          if (act[u]) st[u] = min((int)c.tips[(size_t)id * c.P + p[u]], c.unknown);
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+          for (int x = 0; x < 4; x++)
+            row[u][x] = (R)__ldg((SRC == kM4 ? c.tip_real : c.tip) + st[u] * 4 + x);
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+          for (int x = 0; x < 4; x++) {
+            if constexpr (SRC == kM4) {
+              const float4 r = P[x];
+              v[side][u][x] = fmaf(r.w, row[u][3], fmaf(r.z, row[u][2], fmaf(r.y, row[u][1], fmaf(r.x, row[u][0], 0.f))));
+            } else {
+              double acc = 0.0;
+#pragma unroll
+              for (int i = 0; i < 4; i++) acc = fma(ev[x * 4 + i] * d[i], row[u][i], acc);
+              v[side][u][x] = st[u] == c.unknown ? 1.0 : acc;
+            }
+          }
+        continue;
+      }
+      const bool kept = id == slot;
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+#pragma unroll
+        for (int x = 0; x < 4; x++) row[u][x] = last[u][x];
+        if (kept) {
+          sc[u] += slast[u];
+        } else if (act[u]) {
+          const R *src = part + (size_t)id * c.slot_elems;
+          if constexpr (SRC == kM4) {
+            const float4 r = __ldcg(reinterpret_cast<const float4 *>(src + mix_off<4>(c, p[u], cat)));
+            row[u][0] = r.x, row[u][1] = r.y, row[u][2] = r.z, row[u][3] = r.w;
+          } else {
+            const double2 a = __ldcg(reinterpret_cast<const double2 *>(src + f64_off<4>(c, p[u], cat, 0)));
+            const double2 b = __ldcg(reinterpret_cast<const double2 *>(src + f64_off<4>(c, p[u], cat, 2)));
+            row[u][0] = a.x, row[u][1] = a.y, row[u][2] = b.x, row[u][3] = b.y;
+          }
+          sc[u] += c.scale[(size_t)id * c.slot_scale + (SAFE ? (size_t)p[u] * C + cat : (size_t)p[u])];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          if constexpr (SRC == kM4) {
+            const float4 r = P[x];
+            v[side][u][x] = fmaf(r.w, row[u][3], fmaf(r.z, row[u][2], fmaf(r.y, row[u][1], fmaf(r.x, row[u][0], 0.f))));
+          } else {
+            double acc = 0.0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc = fma(ev[x * 4 + i], row[u][i] * d[i], acc);
+            v[side][u][x] = acc;
+          }
+        }
+    }
+    const bool tiptip = op.l_kind == GEMS_CHILD_TIP && op.r_kind == GEMS_CHILD_TIP;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      // the row's maximum as bits that compare like it (FP64: the high word; NaN counts as zero)
+      int h = 0;
+      if constexpr (SRC == kM4) {
+        float m = 0.f;
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          last[u][x] = v[0][u][x] * v[1][u][x];
+          m = fmaxf(m, last[u][x]);
+        }
+        h = __float_as_int(m);
+      } else {
+        double t[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) t[x] = v[0][u][x] * v[1][u][x];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int x = 0; x < 4; x++) acc = fma(iv[j * 4 + x], t[x], acc);
+          last[u][j] = acc;
+          const int w = __double2hiint(acc) & 0x7fffffff;
+          h = max(h, w > 0x7ff00000 ? 0 : w);
+        }
+      }
+      if (!SAFE) {
+        if (!act[u]) h = 0;
+        for (int q = 1; q < L; q <<= 1) h = max(h, __shfl_xor_sync(0xffffffffu, h, q));
+      }
+      // 2^-256, or 2^-64 as a float
+      const int thr = SRC == kM4 ? 0x1f800000 : 0x2FF00000;
+      if (!tiptip && h < thr && inv0[u]) {
+#pragma unroll
+        for (int x = 0; x < 4; x++) last[u][x] *= (R)(SRC == kM4 ? 0x1p64 : 0x1p256);
+        sc[u] += 1;
+      }
+      slast[u] = sc[u];
+      if (!act[u]) continue;
+      R *dst = part + (size_t)op.dst_slot * c.slot_elems;
+      if constexpr (SRC == kM4) {
+        *reinterpret_cast<float4 *>(dst + mix_off<4>(c, p[u], cat)) =
+            make_float4(last[u][0], last[u][1], last[u][2], last[u][3]);
+      } else {
+        *reinterpret_cast<double2 *>(dst + f64_off<4>(c, p[u], cat, 0)) =
+            make_double2(last[u][0], last[u][1]);
+        *reinterpret_cast<double2 *>(dst + f64_off<4>(c, p[u], cat, 2)) =
+            make_double2(last[u][2], last[u][3]);
+      }
+      uint16_t *scd = c.scale + (size_t)op.dst_slot * c.slot_scale;
+      if (SAFE)
+        scd[(size_t)p[u] * C + cat] = (uint16_t)sc[u];
+      else if (l == 0)
+        scd[p[u]] = (uint16_t)sc[u];
+    }
+    slot = op.dst_slot;
+    __syncwarp();  // NORM: the counter that lane 0 wrote is read by its pattern's lanes
+  }
+}
+
 constexpr int kThreadsT = 256;
 // resident blocks per SM (the registers of two patterns' elements)
 constexpr int ctas_t(int e2) { return e2 <= 2 ? 3 : (e2 <= 5 ? 2 : 1); }
@@ -307,7 +511,7 @@ constexpr int ctas_t(int e2) { return e2 <= 2 ? 3 : (e2 <= 5 ? 2 : 1); }
 template <int SRC, bool SAFE, int E2>
 __global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
     k_terms(DevCtx c, gems_branch br, double t, int L, int flags, unsigned int *ticket,
-            double *out) {
+            double *out, const __grid_constant__ SmallOps ops) {
   extern __shared__ __align__(16) double tab[];
   __shared__ double sh[kThreadsT / 32][2];
   __shared__ bool last;
@@ -317,6 +521,9 @@ __global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
     table_factors(c, j, cof, prop);
     put_tables(t, j, cof, prop, len, flags & kDerv ? 3 : 1, tab);
   }
+  double *small = tab + (flags & kDerv ? 3 : 1) * len;
+  if constexpr (small_form<SRC, E2>())
+    if (ops.n) small_tables<SRC>(c, ops, small);
   __syncthreads();
   const int l = threadIdx.x & (L - 1);
   const long per = blockDim.x / L, step = per * gridDim.x;
@@ -334,6 +541,8 @@ __global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
       f = c.freq[p];
       if (SRC == kMem && (flags & kLnl)) sc = c.scale_all[p];
     }
+    if constexpr (small_form<SRC, E2>())
+      if (ops.n) small_traverse<SRC, SAFE>(c, ops, small, L, l, pu);
     load_theta<SRC, SAFE, E2>(c, br, L, l, pu, th, ms);
     if (flags & kStore) {
 #pragma unroll
@@ -509,7 +718,7 @@ __host__ __device__ constexpr int held_rows() {
 
 template <int SRC, bool SAFE, int E2>
 __global__ void __launch_bounds__(newton_threads(E2), 1)
-    k_newton(DevCtx c, const NewtonArgs a) {
+    k_newton(DevCtx c, const NewtonArgs a, const __grid_constant__ SmallOps ops) {
   constexpr int kThreadsN = newton_threads(E2), kWarps = kThreadsN / 32;
   extern __shared__ __align__(16) double tab[];
   __shared__ __align__(16) double2 recv[2][kMaxCluster * kWarps];
@@ -535,6 +744,17 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
   }
   // the others' barriers are ready once all blocks have been here (waited for below)
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+
+  const double *small = tab + 3 * len;
+  if constexpr (small_form<SRC, E2>())
+    if (ops.n) {
+      small_tables<SRC>(c, ops, tab + 3 * len);
+      __syncthreads();
+    }
+  auto updates = [&](const long (&p)[2]) {
+    if constexpr (small_form<SRC, E2>())
+      if (ops.n) small_traverse<SRC, SAFE>(c, ops, small, L, l, p);
+  };
 
   // theta of this thread's rows: formed and stored (or read), the first ones kept; of each two
   // patterns, even lanes hold the first's +I term and weight and odd lanes the second's
@@ -562,6 +782,7 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
     double v[2][2 * E2];
     int m[2];
     weights(l & 1 ? p[1] : p[0], inva[r / 2], fr[r / 2]);
+    updates(p);
     load_theta<SRC, SAFE, E2>(c, a.br, L, l, p, v, m);
     keep(p, v, m);
 #pragma unroll
@@ -572,6 +793,7 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
       const long p[2] = {b + sub, b + step + sub};
       double v[2][2 * E2];
       int m[2];
+      updates(p);
       load_theta<SRC, SAFE, E2>(c, a.br, L, l, p, v, m);
       keep(p, v, m);
     }
@@ -765,10 +987,29 @@ bool theta_in_kernel(const Session *s) {
   return s->desc.precision == GEMS_PREC_FP64 || s->desc.nstates == 4;
 }
 
+static bool mixed_of(const Session *s) { return s->desc.precision == GEMS_PREC_MIXED; }
+
+// Op lists that a branch call runs in its own launch: few of them, and few enough patterns that
+// the launches around them cost more than the lanes' own loads (from about 2^15 on, the traversal
+// kernels' staged tables and one thread per pattern are the faster way).
+bool small_ops(const Session *s, int nops) {
+  return s->desc.nstates == 4 && s->desc.ncat >= 2 && nops >= 1 && nops <= kSmallOps &&
+         nops * s->desc.ncat <= 64 && s->P <= kSmallPatterns && s->force_shape < 0;
+}
+static SmallOps small_list(const gems_op *ops, int nops) {
+  SmallOps o;
+  std::memset(&o, 0, sizeof(o));
+  o.n = nops;
+  if (nops) std::memcpy(o.op, ops, sizeof(DevOp) * nops);
+  return o;
+}
+
 // br: theta from the branch's partials; null: theta as stored.  The two results are in
 // s->h_result once the stream has completed.
-int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length) {
+int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length,
+                  const gems_op *ops, int nops) {
   DevCtx c = s->ctx();
+  SmallOps o = small_list(ops, nops);
   Split sp = split_of(s->block, s->desc.ncat);
   const Fns f = kernels_for(s, br != nullptr, sp.E2);
   const long per = kThreadsT / sp.L;
@@ -776,10 +1017,11 @@ int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, doubl
   gems_branch b{};
   if (br) b = *br;
   int flags = (store ? kStore : 0) | (lnl ? kLnl : kDerv);
-  const size_t smem = sizeof(double) * 2 * sp.L * sp.E2 * (lnl ? 1 : 3);
+  const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * (lnl ? 1 : 3) +
+                                        small_doubles(nops, s->desc.ncat, mixed_of(s)));
   unsigned int *ticket = s->d_bar;
   double *out = s->h_result;
-  void *args[] = {&c, &b, &length, &sp.L, &flags, &ticket, &out};
+  void *args[] = {&c, &b, &length, &sp.L, &flags, &ticket, &out, &o};
   const int id = lnl ? (br ? 1 : 4) : 3;
   cudaEvent_t ev0;
   if (int st = prof_begin(s, id, &ev0)) return st;
@@ -794,8 +1036,9 @@ double terms_lnl(const Session *s) {
   return std::isfinite(s->h_result[0]) ? s->h_result[0] : s->h_result[1];
 }
 
-int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf) {
-  if (int st = enqueue_terms(s, br, br != nullptr, false, length)) return st;
+int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf,
+                const gems_op *ops, int nops) {
+  if (int st = enqueue_terms(s, br, br != nullptr, false, length, ops, nops)) return st;
   if (int st = sync_session(s)) return st;
   *df = s->h_result[0];
   *ddf = s->h_result[1];
@@ -804,7 +1047,7 @@ int launch_derv(Session *s, const gems_branch *br, double length, double *df, do
 }
 
 int launch_from_buffer(Session *s, double length, double *lnl) {
-  if (int st = enqueue_terms(s, nullptr, false, true, length)) return st;
+  if (int st = enqueue_terms(s, nullptr, false, true, length, nullptr, 0)) return st;
   if (int st = sync_session(s)) return st;
   *lnl = terms_lnl(s);
   return GEMS_OK;
@@ -820,13 +1063,16 @@ int newton_result(Session *s, double *opt_len, int *nevals) {
 }
 
 int launch_newton_async(Session *s, const gems_branch *br, double guess, double min_len,
-                        double max_len, double xacc, int max_steps) {
+                        double max_len, double xacc, int max_steps, const gems_op *ops,
+                        int nops) {
   DevCtx c = s->ctx();
+  SmallOps o = small_list(ops, nops);
   const Split sp = split_of(s->block, s->desc.ncat);
   const Fns f = kernels_for(s, br != nullptr, sp.E2);
   int nsm = 0;
   GEMS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device));
-  const size_t smem = sizeof(double) * 2 * sp.L * sp.E2 * 3;
+  const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * 3 +
+                                        small_doubles(nops, s->desc.ncat, mixed_of(s)));
   const int threads = newton_threads(sp.E2);
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -886,7 +1132,7 @@ int launch_newton_async(Session *s, const gems_branch *br, double guess, double 
   a.slots = reinterpret_cast<ulonglong2 *>(s->d_slots);
   a.tag0 = (unsigned long long)(++s->newton_launches) << 32;
   a.result = s->h_result;
-  void *args[] = {&c, &a};
+  void *args[] = {&c, &a, &o};
   cudaEvent_t ev0;
   if (int st = prof_begin(s, 5, &ev0)) return st;
   GEMS_CUDA(cudaLaunchKernelExC(&cfg, f.newton, args));

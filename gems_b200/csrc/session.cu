@@ -225,12 +225,11 @@ static void free_session(Session *s) {
   }
 }
 
-static int upload_ops(Session *s, const gems_op *ops, int nops) {
+static int check_ops(const Session *s, const gems_op *ops, int nops) {
   if (nops < 0 || nops > s->nops_max) {
     set_error("too many traversal ops");
     return GEMS_ERR_BAD_ARG;
   }
-  if (nops == 0) return GEMS_OK;
   for (int k = 0; k < nops; k++) {
     const gems_op &o = ops[k];
     auto bad_child = [&](int kind, int id) {
@@ -244,6 +243,12 @@ static int upload_ops(Session *s, const gems_op *ops, int nops) {
       return GEMS_ERR_BAD_ARG;
     }
   }
+  return GEMS_OK;
+}
+
+static int upload_ops(Session *s, const gems_op *ops, int nops) {
+  if (int st = check_ops(s, ops, nops)) return st;
+  if (nops == 0) return GEMS_OK;
   // host staging: wait for any kernel still reading the previous op table
   GEMS_CUDA(cudaStreamSynchronize(s->stream));
   s->plan_depth = plan_ops(ops, nops, s->desc.nslots, reinterpret_cast<gems_op *>(s->h_ops));
@@ -302,8 +307,7 @@ static int pattern_granule(const Session *s) {
   }
 }
 
-// the op tables of `nops` uploaded ops, then their traversal over patterns [p0, p1)
-static int run_ops_range(Session *s, const gems_op *ops, int nops, int p0, int p1) {
+static int check_ready(const Session *s) {
   if (!s->model_set) {
     set_error("model not set");
     return GEMS_ERR_STATE;
@@ -312,6 +316,12 @@ static int run_ops_range(Session *s, const gems_op *ops, int nops, int p0, int p
     set_error("tip states invalid (last upload was rejected)");
     return GEMS_ERR_STATE;
   }
+  return GEMS_OK;
+}
+
+// the op tables of `nops` uploaded ops, then their traversal over patterns [p0, p1)
+static int run_ops_range(Session *s, const gems_op *ops, int nops, int p0, int p1) {
+  if (int st = check_ready(s)) return st;
   int st = upload_ops(s, ops, nops);
   if (st) return st;
   switch (traversal_form(s)) {
@@ -344,6 +354,18 @@ static int run_ops(Session *s, const gems_op *ops, int nops) {
   return run_ops_range(s, ops, nops, 0, s->P);
 }
 
+// The node updates of a branch call: run here, or (short lists, small_ops) left to the launch
+// that follows, which is then given the first `*left` of them.
+static int run_branch_ops(Session *s, const gems_op *ops, int nops, int *left) {
+  *left = 0;
+  if (!small_ops(s, nops)) return run_ops(s, ops, nops);
+  if (int st = check_ready(s)) return st;
+  if (int st = check_ops(s, ops, nops)) return st;
+  invalidate_theta(s, ops, nops);
+  *left = nops;
+  return GEMS_OK;
+}
+
 static void copy_pattern_lh(Session *s, double *pattern_lh, double lnl_raw_finite) {
   (void)lnl_raw_finite;
   if (!pattern_lh) return;
@@ -355,12 +377,14 @@ static void copy_pattern_lh(Session *s, double *pattern_lh, double lnl_raw_finit
 }
 
 // the lnL of a branch from its partials
-static int enqueue_branch_lnl(Session *s, const gems_branch *br) {
-  if (theta_in_kernel(s)) return enqueue_terms(s, br, false, true, br->length);
+static int enqueue_branch_lnl(Session *s, const gems_branch *br, const gems_op *ops = nullptr,
+                              int nops = 0) {
+  if (theta_in_kernel(s)) return enqueue_terms(s, br, false, true, br->length, ops, nops);
   return enqueue_theta_mixed(s, br, true, false);
 }
-static int launch_branch_lnl(Session *s, const gems_branch *br, double *lnl) {
-  if (int st = enqueue_branch_lnl(s, br)) return st;
+static int launch_branch_lnl(Session *s, const gems_branch *br, double *lnl,
+                             const gems_op *ops = nullptr, int nops = 0) {
+  if (int st = enqueue_branch_lnl(s, br, ops, nops)) return st;
   if (int st = sync_session(s)) return st;
   *lnl = terms_lnl(s);
   return GEMS_OK;
@@ -902,8 +926,9 @@ int gems_branch_lnl(gems_session *s, const gems_op *ops, int nops, const gems_br
   GEMS_CUDA(cudaSetDevice(s->desc.device));
   int st = check_branch(s, br);
   if (st) return st;
-  if ((st = run_ops(s, ops, nops))) return st;
-  if ((st = launch_branch_lnl(s, br, lnl))) return st;
+  int left = 0;
+  if ((st = run_branch_ops(s, ops, nops, &left))) return st;
+  if ((st = launch_branch_lnl(s, br, lnl, ops, left))) return st;
   copy_pattern_lh(s, pattern_lh, *lnl);
   return GEMS_OK;
 }
@@ -1008,10 +1033,11 @@ int gems_branch_derv(gems_session *s, const gems_op *ops, int nops, const gems_b
                      int compute_theta, double *df, double *ddf, double *df_frac) {
   if (!s || !df || !ddf || (nops > 0 && !ops)) return GEMS_ERR_BAD_ARG;
   GEMS_CUDA(cudaSetDevice(s->desc.device));
+  int left = 0;
   int st = check_branch(s, br);
   if (st) return st;
   if (compute_theta) {
-    if ((st = run_ops(s, ops, nops))) return st;
+    if ((st = run_branch_ops(s, ops, nops, &left))) return st;
     if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
     s->theta_valid = true;
     s->theta_branch = *br;
@@ -1020,7 +1046,7 @@ int gems_branch_derv(gems_session *s, const gems_op *ops, int nops, const gems_b
     return GEMS_ERR_STATE;
   }
   const bool form = compute_theta && theta_in_kernel(s);
-  if ((st = launch_derv(s, form ? br : nullptr, br->length, df, ddf))) return st;
+  if ((st = launch_derv(s, form ? br : nullptr, br->length, df, ddf, ops, left))) return st;
   if (df_frac) {
     GEMS_CUDA(cudaMemcpyAsync(df_frac, s->d_df_frac, sizeof(double) * s->desc.nptn,
                               cudaMemcpyDeviceToHost, s->stream));
@@ -1048,10 +1074,11 @@ int gems_newton_branch_async(gems_session *s, const gems_op *ops, int nops,
   if (!s || (nops > 0 && !ops) || !(min_len >= 0) || !(max_len >= min_len) || max_steps < 1)
     return GEMS_ERR_BAD_ARG;
   GEMS_CUDA(cudaSetDevice(s->desc.device));
+  int left = 0;
   int st = check_branch(s, br);
   if (st) return st;
   if (compute_theta) {
-    if ((st = run_ops(s, ops, nops))) return st;
+    if ((st = run_branch_ops(s, ops, nops, &left))) return st;
     if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
     s->theta_valid = true;
     s->theta_branch = *br;
@@ -1060,7 +1087,7 @@ int gems_newton_branch_async(gems_session *s, const gems_op *ops, int nops,
     return GEMS_ERR_STATE;
   }
   return launch_newton_async(s, compute_theta && theta_in_kernel(s) ? br : nullptr, br->length,
-                             min_len, max_len, xacc, max_steps);
+                             min_len, max_len, xacc, max_steps, ops, left);
 }
 
 int gems_newton_branch_wait(gems_session *s, double *opt_len, int *nevals) {
