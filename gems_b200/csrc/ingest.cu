@@ -15,8 +15,10 @@
 //   assign   per site: pattern id, frequency (integer atomics), the pattern's first site
 //   gather   pattern columns; const   the constant state of each pattern
 // Every loop is bounded (the table has at least twice as many slots as sites).
+#include <algorithm>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "gems_internal.cuh"
@@ -26,11 +28,10 @@ namespace {
 
 constexpr unsigned long long kEmpty = ~0ULL;
 
-__global__ void k_encode(uint8_t *codes, const uint8_t *chars, size_t n, const uint8_t *lut,
-                         unsigned long long *bad) {
+__global__ void k_encode(uint8_t *codes, size_t n, const uint8_t *lut, unsigned long long *bad) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    const uint8_t v = lut[chars[i]];
+    const uint8_t v = lut[codes[i]];
     if (v == 0xFF) atomicMin(bad, (unsigned long long)i);  // first bad position
     codes[i] = v;
   }
@@ -258,10 +259,8 @@ struct gems_ingest {
 extern "C" void gems_ingest_destroy(gems_ingest *g) {
   if (!g) return;
   cudaSetDevice(g->device);
-  cudaFree(g->d_pat);
-  cudaFree(g->d_cc);
-  cudaFree(g->d_count);
-  cudaFree(g->d_sp);
+  cudaFree(g->d_pat);    // and d_cc
+  cudaFree(g->d_count);  // and d_sp
   if (g->st) cudaStreamDestroy(g->st);
   delete g;
 }
@@ -291,16 +290,26 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
   unsigned long long cap = 1;
   while (cap < 2ULL * (unsigned long long)nsites) cap <<= 1;
   const long long nblk = (nsites + 1023) / 1024;
-  // working buffers, freed before returning
-  uint8_t *d_raw = nullptr, *d_codes = nullptr, *d_lut = nullptr;
-  unsigned long long *d_h = nullptr, *d_tab = nullptr, *d_min = nullptr, *d_bad = nullptr;
-  long long *d_grp = nullptr, *d_pid = nullptr, *d_bsum = nullptr, *d_rep = nullptr;
-  unsigned int *d_flag = nullptr;
-  auto release = [&]() {
-    cudaFree(d_raw); cudaFree(d_codes); cudaFree(d_lut); cudaFree(d_h); cudaFree(d_tab);
-    cudaFree(d_min); cudaFree(d_bad); cudaFree(d_grp); cudaFree(d_pid); cudaFree(d_bsum);
-    cudaFree(d_rep); cudaFree(d_flag);
+  // working buffers, one allocation (each cudaMalloc and cudaFree costs 0.1 ms and more, 14 pairs
+  // of them were half of a 256 x 200,000 ingest's 11 ms), freed before returning
+  size_t bytes = 0;
+  auto take = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
   };
+  const size_t o_codes = take(cells), o_lut = take(256);
+  const size_t o_h = take(sizeof(unsigned long long) * nsites);
+  const size_t o_tab = take(sizeof(unsigned long long) * cap);
+  const size_t o_min = take(sizeof(unsigned long long) * cap);
+  const size_t o_bad = take(sizeof(unsigned long long));
+  const size_t o_grp = take(sizeof(long long) * nsites);
+  const size_t o_pid = take(sizeof(long long) * nsites);
+  const size_t o_bsum = take(sizeof(long long) * (nblk + 1));
+  const size_t o_rep = take(sizeof(long long) * nsites);
+  const size_t o_flag = take(sizeof(unsigned int) * nsites);
+  uint8_t *work = nullptr;
+  auto release = [&]() { cudaFree(work); };
   auto fail = [&](cudaError_t e, const char *what) {
     const int code = cuda_status(e, what);
     release();
@@ -308,25 +317,21 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
     return code;
   };
   cudaError_t e;
-#define ALLOC(p, bytes) \
-  if ((e = cudaMalloc((void **)&(p), (bytes))) != cudaSuccess) return fail(e, "cudaMalloc " #p);
-  ALLOC(d_codes, cells);
-  if (!encoded) {
-    ALLOC(d_raw, cells);
-    ALLOC(d_lut, 256);
-  }
-  ALLOC(d_h, sizeof(unsigned long long) * nsites);
-  ALLOC(d_tab, sizeof(unsigned long long) * cap);
-  ALLOC(d_min, sizeof(unsigned long long) * cap);
-  ALLOC(d_bad, sizeof(unsigned long long));
-  ALLOC(d_grp, sizeof(long long) * nsites);
-  ALLOC(d_pid, sizeof(long long) * nsites);
-  ALLOC(d_bsum, sizeof(long long) * (nblk + 1));
-  ALLOC(d_rep, sizeof(long long) * nsites);
-  ALLOC(d_flag, sizeof(unsigned int) * nsites);
-  ALLOC(g->d_count, sizeof(unsigned int) * nsites);
-  ALLOC(g->d_sp, sizeof(int) * nsites);
-#undef ALLOC
+  if ((e = cudaMalloc((void **)&work, bytes)) != cudaSuccess) return fail(e, "cudaMalloc ingest");
+  if ((e = cudaMalloc((void **)&g->d_count, (sizeof(unsigned int) + sizeof(int)) * nsites)) !=
+      cudaSuccess)
+    return fail(e, "cudaMalloc counts");
+  g->d_sp = reinterpret_cast<int *>(g->d_count + nsites);
+  uint8_t *d_codes = work + o_codes, *d_lut = work + o_lut;
+  auto *d_h = reinterpret_cast<unsigned long long *>(work + o_h);
+  auto *d_tab = reinterpret_cast<unsigned long long *>(work + o_tab);
+  auto *d_min = reinterpret_cast<unsigned long long *>(work + o_min);
+  auto *d_bad = reinterpret_cast<unsigned long long *>(work + o_bad);
+  auto *d_grp = reinterpret_cast<long long *>(work + o_grp);
+  auto *d_pid = reinterpret_cast<long long *>(work + o_pid);
+  auto *d_bsum = reinterpret_cast<long long *>(work + o_bsum);
+  auto *d_rep = reinterpret_cast<long long *>(work + o_rep);
+  auto *d_flag = reinterpret_cast<unsigned int *>(work + o_flag);
   if ((e = cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(e, "cudaStreamCreate");
   cudaStream_t st = g->st;
@@ -336,11 +341,11 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
   if (!encoded) {
     uint8_t lut[256];
     build_lut(nstates, lut);
-    if ((e = cudaMemcpyAsync(d_raw, seqs, cells, cudaMemcpyHostToDevice, st)) ||
+    if ((e = cudaMemcpyAsync(d_codes, seqs, cells, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(d_lut, lut, 256, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(d_bad, &bad, sizeof(bad), cudaMemcpyHostToDevice, st)))
       return fail(e, "ingest upload");
-    k_encode<<<1184, T, 0, st>>>(d_codes, d_raw, cells, d_lut, d_bad);
+    k_encode<<<1184, T, 0, st>>>(d_codes, cells, d_lut, d_bad);
     if ((e = cudaGetLastError()) ||
         (e = cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, st)) ||
         (e = cudaStreamSynchronize(st)))
@@ -374,9 +379,9 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
       (e = cudaStreamSynchronize(st)))
     return fail(e, "ingest compress");
   g->npat = npat;
-  if ((e = cudaMalloc((void **)&g->d_pat, (size_t)ntaxa * npat)) != cudaSuccess ||
-      (e = cudaMalloc((void **)&g->d_cc, (size_t)npat)) != cudaSuccess)
+  if ((e = cudaMalloc((void **)&g->d_pat, (size_t)(ntaxa + 1) * npat)) != cudaSuccess)
     return fail(e, "cudaMalloc patterns");
+  g->d_cc = g->d_pat + (size_t)ntaxa * npat;
   const unsigned gp = (unsigned)((npat + T - 1) / T);
   k_gather<<<gp, T, 0, st>>>(d_codes, ntaxa, nsites, npat, d_rep, g->d_pat);
   k_const<<<gp, T, 0, st>>>(g->d_pat, ntaxa, npat, nstates, g->d_cc);
@@ -387,11 +392,36 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
   return GEMS_OK;
 }
 
+// Writes one byte of every page of a destination that a copy will fill.  A caller's fresh array
+// has no pages yet, and a device copy into it faults them in one by one (43 MB: 10 ms instead of
+// 2.5); a few threads take the faults side by side.
+static void touch_pages(uint8_t *p, size_t n) {
+  constexpr size_t kPage = 4096, kLeast = 4u << 20;
+  if (n < kLeast) return;
+  const size_t per = 2u << 20;
+  const int most = (int)std::min<size_t>(8, std::thread::hardware_concurrency());
+  const int nt = (int)std::min<size_t>((size_t)std::max(1, most), n / per);
+  auto touch = [p, n, nt](int t) {
+    const size_t a = n / nt * t, b = t + 1 == nt ? n : n / nt * (t + 1);
+    for (size_t i = a; i < b; i += kPage) *(volatile uint8_t *)(p + i) = 0;
+    *(volatile uint8_t *)(p + b - 1) = 0;
+  };
+  std::vector<std::thread> ts;
+  int t = 1;
+  try {
+    for (; t < nt; t++) ts.emplace_back(touch, t);
+  } catch (...) {  // no more threads: the copy takes the remaining faults
+  }
+  touch(0);
+  for (std::thread &x : ts) x.join();
+}
+
 extern "C" int gems_ingest_read(gems_ingest *g, uint8_t *patterns, double *weights,
                                 int *site_pattern, uint8_t *const_char) {
   if (!g) return GEMS_ERR_BAD_ARG;
   GEMS_CUDA(cudaSetDevice(g->device));
   std::vector<unsigned int> cnt((size_t)g->npat);
+  if (patterns) touch_pages(patterns, (size_t)g->ntaxa * g->npat);
   if (patterns)
     GEMS_CUDA(cudaMemcpyAsync(patterns, g->d_pat, (size_t)g->ntaxa * g->npat,
                               cudaMemcpyDeviceToHost, g->st));
