@@ -535,11 +535,13 @@ size_t tc61_smem() { return 4 * (size_t)kATile + 2 * (size_t)kBSide + sizeof(Tc6
 // and the epilogue).
 //   warps 0-3, split: one thread per pattern row.  Waits for the operand tiles of step s in
 //     landing buffer s&1 and splits each internal child's row: hi -> TMEM A_hi[s&1][side], lo
-//     written back in place (the landing buffer is then the lo operand of the MMAs).
+//     written back in place (the landing buffer is then the lo operand of the MMAs).  A tip
+//     child's message, a row of the tip table in the side's landing buffer, goes into the side's
+//     accumulator D[s&1], once the epilogue of step s-2 has read that.
 //   warps 4-11, epilogue: two threads per pattern row, 32 states each (warps w and w+4 share
-//     TMEM lane quadrant w%4).  A tip child's message is its tip table row, read before the
-//     wait; waits for the MMAs of step s, reads D[s&1] and frees it; products, the row maximum
-//     over both halves (exchanged in shared memory), SAFE rescaling.  The rows go into a 32 KB
+//     TMEM lane quadrant w%4).  Waits for the MMAs of step s (and the split's tip messages),
+//     reads D[s&1] and frees it; products, the row maximum over both halves (exchanged in shared
+//     memory), SAFE rescaling.  The rows go into a 32 KB
 //     staging buffer, so that no per-thread global store sits in the SM's memory path beside
 //     the copies and MMAs.  The epilogue is the longest part of a step, so it has the most
 //     warps.
@@ -547,9 +549,9 @@ size_t tc61_smem() { return 4 * (size_t)kATile + 2 * (size_t)kBSide + sizeof(Tc6
 //     buffer the epilogue may fill it again, and once it has completed the number of steps
 //     stored is published.
 //   warp 12, copies: the operand tiles (tip sides: the 16.5 KB tip table) of step s into landing
-//     buffer s&1, once the MMAs and the epilogue's tip reads of step s-2 are done with it and
-//     every step that wrote one of those children has published its stores; the B images of
-//     internal sides, in step order, into a ring of two 32 KB slots.
+//     buffer s&1, once the MMAs of step s-2 are done with it and every step that wrote one of
+//     those children has published its stores; the B images of internal sides, in step order,
+//     into a ring of two 32 KB slots.
 //   warp 13, MMAs: step s into D[s&1] once its split is done, its B images have landed and the
 //     epilogue of step s-2 has read D[s&1]; a commit per side frees its ring slot, a commit per
 //     step signals the epilogue and the copies.
@@ -559,10 +561,12 @@ size_t tc61_smem() { return 4 * (size_t)kATile + 2 * (size_t)kBSide + sizeof(Tc6
 // the form above: the same bits.  Every wait is bounded and also gives up once another role has
 // failed (err); on failure the copy, MMA and store warps wait (bounded) for what they have in
 // flight before TMEM and shared memory are released.
-// Tip rows were read from the table in global memory at first, 256 L1 wavefronts for a warp's 32
-// rows of 128 bytes: half of the launch's L1 cycles.  From a landing buffer the evaluation of 32
-// candidate models (200 taxa, 3,780 patterns, +G4) takes 15.2 ms instead of 17.8; 16 models with
-// 8 categories 15.7 instead of 18.5.
+// Tip rows were read by the epilogue from the table in global memory at first, 256 L1 wavefronts
+// for a warp's 32 rows of 128 bytes, half of the launch's L1 cycles.  The evaluation of 32
+// candidate models (200 taxa, 3,780 patterns, +G4; traversal, op tables and branch terms) took
+// 17.6 ms then, 14.5 with the tables in landing buffers and the rows still read by the epilogue
+// (bank conflicts of random rows on the longest role), 12.6 with the split warps, which have the
+// time, moving them into the accumulators; 16 models with 8 categories 18.5, 15.7 and 13.4 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int kWsThreads = 480;
 static_assert(kTipBytes61 % 16 == 0 && kTipBytes61 <= kATile, "a tip table fits a landing buffer");
@@ -643,19 +647,48 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     // ---- split
     const int row = t;
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+    const long p = (long)tile * kTile + row;
+    const bool act = p < c.P;
     StepIt it{0, 0, ops[0]};
+    int st[2] = {0, 0};
+    bool had_tip[2] = {false, false};  // the epilogue of the last step on this parity reads
+                                       // split_done, which must not run two phases ahead of it
     for (int s = 0; s < nsteps; s++) {
-      const int b = s & 1;
-      const bool inL = it.op.l_kind == GEMS_CHILD_PARTIAL, inR = it.op.r_kind == GEMS_CHILD_PARTIAL;
-      if (__any_sync(0xffffffffu, !ws_wait(sptr(&ctl->full_land[b]), (s >> 1) & 1, err))) {
+      const int b = s & 1, u = s >> 1;
+      const bool in[2] = {it.op.l_kind == GEMS_CHILD_PARTIAL, it.op.r_kind == GEMS_CHILD_PARTIAL};
+      if (it.cat == 0) {  // tip state codes of a new op
+        st[0] = in[0] || !act ? 0 : min((int)c.tips[(size_t)it.op.l_id * c.P + p], kN);
+        st[1] = in[1] || !act ? 0 : min((int)c.tips[(size_t)it.op.r_id * c.P + p], kN);
+      }
+      // the step's tiles and tip tables have come; tip messages: D[b] has been read
+      bool ok = ws_wait(sptr(&ctl->full_land[b]), u & 1, err);
+      const bool tip = !(in[0] && in[1]);
+      if ((tip || had_tip[b]) && u >= 1)
+        ok = ok && ws_wait(sptr(&ctl->epi_done[b]), (u - 1) & 1, err);
+      had_tip[b] = tip;
+      if (__any_sync(0xffffffffu, !ok)) {
         ws_fail(err, flag);
         break;
       }
       fence_after();
 #pragma unroll
       for (int side = 0; side < 2; side++) {
-        if (!(side ? inR : inL)) continue;
-        float4 *a4 = reinterpret_cast<float4 *>(land + (size_t)(2 * b + side) * kATile);
+        unsigned char *buf = land + (size_t)(2 * b + side) * kATile;
+        if (!in[side]) {
+          const float4 *tr = reinterpret_cast<const float4 *>(buf + (size_t)st[side] * kTipRow61 * 4);
+#pragma unroll
+          for (int hh = 0; hh < 2; hh++) {
+            float h[32];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const float4 q = tr[8 * hh + i];
+              h[4 * i] = q.x, h[4 * i + 1] = q.y, h[4 * i + 2] = q.z, h[4 * i + 3] = q.w;
+            }
+            tmem_st32(tmem + lane_off + (uint32_t)(b * 128 + side * kNP + 32 * hh), h);
+          }
+          continue;
+        }
+        float4 *a4 = reinterpret_cast<float4 *>(buf);
 #pragma unroll
         for (int hh = 0; hh < 2; hh++) {
           float h[32];
@@ -689,56 +722,30 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     const bool act = p < c.P;
     const bool inv0 = act ? c.invar[p] == 0.0 : false;
     StepIt it{0, 0, ops[0]};
-    int st_l = 0, st_r = 0;
     bool stale_prev = false;  // the previous step's staging wait failed
     for (int s = 0; s < nsteps; s++) {
       const int b = s & 1;
       const DevOp op = it.op;
       const bool inL = op.l_kind == GEMS_CHILD_PARTIAL, inR = op.r_kind == GEMS_CHILD_PARTIAL;
-      if (it.cat == 0 && act) {  // tip state codes of a new op
-        st_l = inL ? 0 : c.tips[(size_t)op.l_id * c.P + p];
-        st_r = inR ? 0 : c.tips[(size_t)op.r_id * c.P + p];
-      }
       int scl = 0, scr = 0;
       if (act) {
         if (inL) scl = c.scale[(size_t)op.l_id * c.slot_scale + (size_t)p * C + it.cat];
         if (inR) scr = c.scale[(size_t)op.r_id * c.slot_scale + (size_t)p * C + it.cat];
       }
-      // messages: a tip child's from its row of the table in the side's landing buffer (read
-      // before the wait for the MMAs), an internal child's from its accumulator
+      // both messages are in D[b]: an internal child's by the MMAs, a tip child's by the split
       uint32_t rm[2][32];
-      bool late = false;
-      if (!inL || !inR)
-        late = __any_sync(0xffffffffu, !ws_wait(sptr(&ctl->full_land[b]), (s >> 1) & 1, err));
-#pragma unroll
-      for (int side = 0; side < 2; side++) {
-        if (side ? inR : inL) continue;
-        const int st = side ? st_r : st_l;
-        const float4 *tr = reinterpret_cast<const float4 *>(land + (size_t)(2 * b + side) * kATile +
-                                                            (size_t)(st < kN ? st : kN) *
-                                                                kTipRow61 * 4) + 8 * half;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const float4 q = tr[i];
-          rm[side][4 * i] = __float_as_uint(q.x);
-          rm[side][4 * i + 1] = __float_as_uint(q.y);
-          rm[side][4 * i + 2] = __float_as_uint(q.z);
-          rm[side][4 * i + 3] = __float_as_uint(q.w);
-        }
-      }
-      const bool bad =
-          __any_sync(0xffffffffu, !ws_wait(sptr(&ctl->mma_done[b]), (s >> 1) & 1, err)) || late;
+      bool came = ws_wait(sptr(&ctl->mma_done[b]), (s >> 1) & 1, err);
+      if (!(inL && inR)) came = came && ws_wait(sptr(&ctl->split_done[b]), (s >> 1) & 1, err);
+      const bool bad = __any_sync(0xffffffffu, !came);
       float v[32];
       if (!bad) {
         fence_after();
 #pragma unroll
         for (int side = 0; side < 2; side++)
-          if (side ? inR : inL)
-            tmem_ld32(tmem + lane_off + (uint32_t)(b * 128 + side * kNP + 32 * half), rm[side]);
+          tmem_ld32(tmem + lane_off + (uint32_t)(b * 128 + side * kNP + 32 * half), rm[side]);
 #pragma unroll
-        for (int side = 0; side < 2; side++)
-          if (side ? inR : inL) tmem_ld32_wait(rm[side]);
-        // D[b] and the tip rows have been read: the MMAs and copies of step s+2 may overwrite them
+        for (int side = 0; side < 2; side++) tmem_ld32_wait(rm[side]);
+        // D[b] has been read: step s+2 may overwrite it
         fence_before();
         mbar_arrive(sptr(&ctl->epi_done[b]));
         float mx = 0.f;
@@ -822,20 +829,17 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       int nimg = 0;
       bool ok = true;
       bool land_armed[2] = {false, false}, slot_armed[kWsSlots] = {};
-      bool had_tip[2] = {false, false};  // the last step in a landing buffer left a tip table there
       uint32_t land_par[2] = {0, 0}, slot_par[kWsSlots] = {};
       for (int s = 0; s < nsteps && ok; s++) {
         const int b = s & 1, u = s >> 1;
         const DevOp &op = it.op;
         const bool in[2] = {op.l_kind == GEMS_CHILD_PARTIAL, op.r_kind == GEMS_CHILD_PARTIAL};
         const int id[2] = {op.l_id, op.r_id};
-        // landing buffer b: the MMAs of step s-2 have read it, and the epilogue its tip tables
-        if (u >= 1 && (!ws_wait(sptr(&ctl->mma_done[b]), (u - 1) & 1, err) ||
-                       (had_tip[b] && !ws_wait(sptr(&ctl->epi_done[b]), (u - 1) & 1, err)))) {
+        // landing buffer b: the split and the MMAs of step s-2 have read it
+        if (u >= 1 && !ws_wait(sptr(&ctl->mma_done[b]), (u - 1) & 1, err)) {
           ok = false;
           break;
         }
-        had_tip[b] = !in[0] || !in[1];
         // the children's rows of this category: stored by the step that wrote them (an op at
         // most three back is waited for exactly, older ones by the step four ops back)
         int need = 0;
