@@ -411,13 +411,13 @@ class Session:
         _check(self.lib.gems_set_rates(self.handle, _dptr(r), _dptr(p)), "gems_set_rates")
 
     def set_tensor_cores(self, on=True):
-        """61-state mixed SAFE traversal on tcgen05 split-TF32 products (default) or FP32 CUDA
-        cores (the 20-state one runs in FP32 either way)."""
+        """20-state mixed traversal on tcgen05 split-TF32 products (default) or FP32 CUDA
+        cores."""
         _check(self.lib.gems_session_set_option(self.handle, 1, int(on)), "set_option")
 
     def set_tc20_halves(self, on=True):
-        """Accepted and without effect: the mixed 20-state traversal has one schedule
-        (GEMS_OPT_TC20_HALVES)."""
+        """20-state tcgen05 traversal at two CTAs per SM in half-steps (GEMS_OPT_TC20_HALVES);
+        same values bit for bit."""
         _check(self.lib.gems_session_set_option(self.handle, 5, int(on)), "set_option")
 
     def set_tc61_roles(self, on=True):

@@ -199,10 +199,9 @@ struct Session {
   // pinned host staging
   DevOp *h_ops = nullptr;
   double *h_result = nullptr;
-  int *h_status = nullptr;  // written by a kernel whose bounded wait expired (sync_session)
   int nred = 0;  // size of d_red in doubles
   std::vector<double> h_evec, h_inv;  // host copy of the eigenvectors in use
-  // tensor-core path (61 states, mixed SAFE)
+  // tensor-core path (20 states, mixed): per-op table stride in floats
   bool tc_enabled = true;
   // FP64 61-state traversal as register-tiled GEMMs (else the per-row kernel)
   bool g61_enabled = true;
@@ -210,6 +209,7 @@ struct Session {
   bool autotune = true;
   int force_shape = -1;  // >= 0: that launch shape, no tuning (comparisons)
   int newton_share = 1;  // the Newton kernel takes at most 1/newton_share of the GPU
+  bool tc20_halves = false;  // 20-state tcgen05 traversal at two CTAs per SM, in half-steps
   bool tc61_roles = true;    // 61-state tcgen05 traversal with split / MMA / epilogue warp roles
   size_t op_stride_tc = 0;
   // FP32 partials stored tile-major (20- and 61-state mixed forms); elements per slot
@@ -231,9 +231,6 @@ struct Session {
 
 // tip bytes into a session (host or device source), checked on the device (session.cu)
 int load_tips(Session *s, const uint8_t *src, size_t src_pitch, cudaMemcpyKind kind);
-
-// waits for the session's stream; GEMS_ERR_TIMEOUT if a kernel's bounded wait expired
-int sync_session(Session *s);
 
 // brackets a launch with timing events when profiling is on
 int prof_begin(Session *s, int kernel, cudaEvent_t *a);
@@ -299,12 +296,12 @@ int traverse_v2_shape(const Session *s, int *patterns_per_group, int *blocks_per
 int launch_prep_ops_f20(Session *s, int nops);
 int launch_traverse_f20(Session *s, int nops, int p0, int p1);
 const void *traverse_f20_kernel(const Session *s, int *threads, int *patterns);
-// mixed 20-state traversal (kernels_m20.cu): floats of an op's tables, op tables, traversal, and
-// the kernel with its threads, patterns and shared memory per CTA (null: does not fit)
-size_t m20_op_floats(int ncat, int unknown);
-const void *traverse_m20_kernel(const Session *s, int *threads, int *patterns, size_t *smem);
-int launch_prep_ops_m20(Session *s, int nops);
-int launch_traverse_m20(Session *s, int nops, int p0, int p1);
+// tcgen05 split-TF32 traversal for 20 states (kernels_tc.cu)
+size_t tc20_op_floats(int ncat, int unknown);
+bool tc20_supported(const Session *s);
+int launch_prep_ops_tc20(Session *s, int nops);
+// p0 a multiple of 128, p1 a multiple of 128 or P
+int launch_traverse_tc20(Session *s, int nops, int p0, int p1);
 // tcgen05 split-TF32 traversal for 61 states, SAFE (kernels_tc61.cu)
 size_t tc61_op_floats(int ncat);
 bool tc61_supported(const Session *s);

@@ -1039,7 +1039,7 @@ double terms_lnl(const Session *s) {
 int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf,
                 const gems_op *ops, int nops) {
   if (int st = enqueue_terms(s, br, br != nullptr, false, length, ops, nops)) return st;
-  if (int st = sync_session(s)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
   *df = s->h_result[0];
   *ddf = s->h_result[1];
   if (!std::isfinite(*df)) *df = *ddf = 0.0;  // phylokernelnew.h:2646-2649
@@ -1048,7 +1048,7 @@ int launch_derv(Session *s, const gems_branch *br, double length, double *df, do
 
 int launch_from_buffer(Session *s, double length, double *lnl) {
   if (int st = enqueue_terms(s, nullptr, false, true, length, nullptr, 0)) return st;
-  if (int st = sync_session(s)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
   *lnl = terms_lnl(s);
   return GEMS_OK;
 }
@@ -1056,7 +1056,7 @@ int launch_from_buffer(Session *s, double length, double *lnl) {
 size_t newton_slot_bytes() { return sizeof(ulonglong2) * 2 * kMaxClusters * kSlotStride; }
 
 int newton_result(Session *s, double *opt_len, int *nevals) {
-  if (int st = sync_session(s)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
   *opt_len = s->h_result[0];
   *nevals = (int)s->h_result[1];
   return (int)s->h_result[2];

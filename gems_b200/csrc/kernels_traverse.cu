@@ -1,5 +1,5 @@
-// kernels_traverse.cu -- whole-traversal kernels for 4-state models (FP64 and mixed), and the
-// dispatch of 4 and 20 states (20 states: kernels_f20.cu, kernels_m20.cu).
+// kernels_traverse.cu -- whole-traversal kernels for 4-state models (FP64 and mixed) and the mixed
+// 20-state form on CUDA cores; the dispatch of both state counts (FP64, 20 states: kernels_f20.cu).
 //
 // One CTA owns a tile of patterns and runs every node update of the traversal over it, in
 // postorder; a pattern stays with one lane group for all ops, so a child written by an earlier
@@ -253,9 +253,129 @@ __global__ void k_prep_ops_mix(DevCtx c, const DevOp *ops, float *tab, size_t st
     leaf[idx] = acc;
   }
 }
+
+template <int N, bool SAFE>
+__device__ __forceinline__ void msg_mix(const DevCtx &c, int kind, int id,
+                                        const float *__restrict__ Pm,
+                                        const float *__restrict__ leaf, long p, int gl,
+                                        float (&v)[N], int &s) {
+  const int C = c.C;
+  if (kind == GEMS_CHILD_TIP) {
+    const int st = min((int)c.tips[(size_t)id * c.P + p], c.unknown);
+    const float *lt = leaf + (size_t)st * c.block + gl * N;
+#pragma unroll
+    for (int x = 0; x < N; x++) v[x] = __ldg(lt + x);
+    s = 0;
+  } else {
+    const float *src = static_cast<const float *>(c.partials) + (size_t)id * c.slot_elems +
+                       mix_off<N>(c, p, gl);
+    const int cs = mix_cs<N>();
+    float L[N];
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N / 4; i++) {
+        const float4 t = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)i * cs));
+        L[4 * i] = t.x;
+        L[4 * i + 1] = t.y;
+        L[4 * i + 2] = t.z;
+        L[4 * i + 3] = t.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; i++) L[i] = __ldcg(src + i);
+    }
+#pragma unroll
+    for (int x = 0; x < N; x++) {
+      const float *row = Pm + ((size_t)x * C + gl) * N;
+      float pr[N];
+      if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N / 4; i++) {
+          const float4 t = __ldg(reinterpret_cast<const float4 *>(row) + i);
+          pr[4 * i] = t.x;
+          pr[4 * i + 1] = t.y;
+          pr[4 * i + 2] = t.z;
+          pr[4 * i + 3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int y = 0; y < N; y++) pr[y] = __ldg(row + y);
+      }
+      float acc = 0.f;
+#pragma unroll
+      for (int y = 0; y < N; y++) acc = fmaf(pr[y], L[y], acc);
+      v[x] = acc;
+    }
+    const uint16_t *sc = c.scale + (size_t)id * c.slot_scale;
+    s = SAFE ? sc[(size_t)p * C + gl] : sc[p];
+  }
+}
+
+// 20 states on CUDA cores (4 states run k_traverse_mix4)
+template <int N, bool SAFE>
+__global__ void __launch_bounds__(kThreads, 1) k_traverse_mix(DevCtx c, const DevOp *__restrict__ ops,
+                                                           int nops, const float *__restrict__ tab,
+                                                           size_t stride_f, int p0, int p1) {
+  const int G = c.G;
+  const int gl = threadIdx.x & (G - 1);
+  const long p = p0 + ((long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const bool act = p < p1 && gl < c.C;
+  const int C = c.C;
+  const size_t nnC = (size_t)N * N * C;
+  float *part = static_cast<float *>(c.partials);
+  __shared__ int4 s_ops[kOpChunk];
+  for (int k = 0; k < nops; k++) {
+    if ((k & (kOpChunk - 1)) == 0) stage_ops(ops, k, nops, s_ops);
+    const OpIds op = staged_op(s_ops, k & (kOpChunk - 1));
+    const float *tk = tab + (size_t)k * stride_f;
+    const bool tiptip = op.l_kind == GEMS_CHILD_TIP && op.r_kind == GEMS_CHILD_TIP;
+    float out[N];
+    float lh_max = 0.f;
+    int sl = 0, sr = 0;
+    if (act) {
+      float vl[N], vr[N];
+      msg_mix<N, SAFE>(c, op.l_kind, op.l_id, tk, tk + 2 * nnC, p, gl, vl, sl);
+      msg_mix<N, SAFE>(c, op.r_kind, op.r_id, tk + nnC,
+                       tk + 2 * nnC + (size_t)(c.unknown + 1) * c.block, p, gl, vr, sr);
+#pragma unroll
+      for (int x = 0; x < N; x++) {
+        out[x] = vl[x] * vr[x];
+        lh_max = fmaxf(lh_max, out[x]);
+      }
+    }
+    if (!SAFE) lh_max = group_maxf(lh_max, G);
+    int s_out = sl + sr;
+    if (act) {
+      if (!tiptip && lh_max < kScaleThrF && c.invar[p] == 0.0) {
+#pragma unroll
+        for (int x = 0; x < N; x++) out[x] *= 18446744073709551616.0f;  // 2^64
+        s_out += 1;
+      }
+      float *dst = part + (size_t)op.dst_slot * c.slot_elems + mix_off<N>(c, p, gl);
+      if constexpr (N % 4 == 0) {
+        const int cs = mix_cs<N>();
+#pragma unroll
+        for (int i = 0; i < N / 4; i++)
+          *reinterpret_cast<float4 *>(dst + (size_t)i * cs) =
+              make_float4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) dst[i] = out[i];
+      }
+      uint16_t *sc = c.scale + (size_t)op.dst_slot * c.slot_scale;
+      if (SAFE)
+        sc[(size_t)p * C + gl] = (uint16_t)s_out;
+      else if (gl == 0)
+        sc[p] = (uint16_t)s_out;
+    }
+    __syncwarp();
+  }
+}
+
 // 4 states: the kernel is latency-bound on its child loads.  Each lane group handles PP
 // patterns (at B blocks per SM), kThreads / G apart, so that a warp has the child loads of all of them in flight at
-// once and loads each P row once for all of them; same arithmetic, in the same order.  Measured on the 512-taxon, 1M-pattern case: one pattern per group
+// once and loads each P row once for all of them; same arithmetic, in the same order, as
+// msg_mix / k_traverse_mix.  Measured on the 512-taxon, 1M-pattern case: one pattern per group
 // at 8 blocks per SM (32 registers) 14.8 ms; two at 5 blocks (48 registers) 12.6 ms; two at 4
 // or 6 blocks 14.8 / 12.7 ms; four at 3 blocks 12.8 ms.  The variant in use is picked by the
 // tuner below; every (PP, B) gives the same values.
@@ -1467,9 +1587,8 @@ bool traverse_v2_supported(const Session *s) {
 
 int launch_prep_ops_v2(Session *s, int nops) {
   if (nops <= 0) return GEMS_OK;
-  if (s->desc.nstates == 20)
-    return s->desc.precision == GEMS_PREC_FP64 ? launch_prep_ops_f20(s, nops)
-                                               : launch_prep_ops_m20(s, nops);
+  if (s->desc.precision == GEMS_PREC_FP64 && s->desc.nstates == 20)
+    return launch_prep_ops_f20(s, nops);
   DevCtx c = s->ctx();
   if (s->desc.precision == GEMS_PREC_MIXED) {
     const size_t smem = sizeof(double) * s->block;
@@ -1508,7 +1627,7 @@ int traverse_v2_wave_patterns(const Session *s) {
       return 0;
     }
   } else if (mixed) {
-    if (!(fn = traverse_m20_kernel(s, &threads, &per_block, &smem))) return 0;
+    fn = safe ? (const void *)k_traverse_mix<20, true> : (const void *)k_traverse_mix<20, false>;
   } else {
     fn = traverse_f20_kernel(s, &threads, &per_block);
   }
@@ -1549,11 +1668,23 @@ int launch_traverse_v2(Session *s, int nops, int p0, int p1) {
   cudaEvent_t ev0;
   if (int st = prof_begin(s, 0, &ev0)) return st;
   int st = GEMS_OK;
-  const bool mixed = s->desc.precision == GEMS_PREC_MIXED;
-  if (s->desc.nstates == 4)
-    st = mixed ? traverse4(s, true, nops, p0, p1, nullptr) : launch_f64_4(s, nops, p0, p1);
-  else
-    st = mixed ? launch_traverse_m20(s, nops, p0, p1) : launch_traverse_f20(s, nops, p0, p1);
+  if (s->desc.precision == GEMS_PREC_MIXED) {
+    DevCtx c = s->ctx();
+    const int grid = grid_for(s, p0, p1);
+    const bool safe = s->desc.scaling == GEMS_SCALE_SAFE;
+    const float *tab = reinterpret_cast<const float *>(s->d_opmats);
+    if (s->desc.nstates == 4) {
+      st = traverse4(s, true, nops, p0, p1, nullptr);
+    } else {
+      if (safe) k_traverse_mix<20, true><<<grid, kThreads, 0, s->stream>>>(c, s->d_ops, nops, tab, s->op_stride, p0, p1);
+      else k_traverse_mix<20, false><<<grid, kThreads, 0, s->stream>>>(c, s->d_ops, nops, tab, s->op_stride, p0, p1);
+      s->launches++;
+      GEMS_CUDA(cudaGetLastError());
+    }
+  } else {
+    st = s->desc.nstates == 4 ? launch_f64_4(s, nops, p0, p1)
+                              : launch_traverse_f20(s, nops, p0, p1);
+  }
   if (st) return st;
   return prof_end(s, 0, ev0);
 }

@@ -55,15 +55,6 @@ DevCtx Session::ctx() const {
   return c;
 }
 
-int sync_session(Session *s) {
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
-  const int st = *(volatile int *)s->h_status;
-  if (!st) return GEMS_OK;
-  *s->h_status = 0;
-  set_error("a kernel's bounded wait expired");
-  return st;
-}
-
 static cudaEvent_t prof_event(Session *s) {
   cudaEvent_t e = nullptr;
   if (!s->prof_free.empty()) {
@@ -145,9 +136,9 @@ static Sizes compute_sizes(const gems_session_desc &d) {
   z.theta_bytes = P * blk * sizeof(double) + 4 * P * sizeof(double);
   z.nops_max = d.ntaxa + 8;
   z.op_stride = 2 * (size_t)d.ncat * d.nstates * d.nstates + 2 * (size_t)(unk + 1) * blk;
-  if (d.nstates == 20 && d.precision == GEMS_PREC_MIXED) {
-    // tables of floats share the buffer
-    const size_t need = (m20_op_floats(d.ncat, unk) + 1) / 2;
+  if (d.nstates == 20 && d.precision == GEMS_PREC_MIXED && d.ncat <= 4) {
+    // the tensor-core tables (floats) share the buffer
+    const size_t need = (tc20_op_floats(d.ncat, unk) + 1) / 2;
     if (z.op_stride < need) z.op_stride = need;
   }
   if (d.nstates == 61 && d.precision == GEMS_PREC_MIXED && d.scaling == GEMS_SCALE_SAFE) {
@@ -284,9 +275,10 @@ static void invalidate_theta(Session *s, const gems_op *ops, int nops) {
 
 // The traversal kernel family a session uses, and the pattern granule a pattern range of it
 // must respect (lower bound a multiple of it; upper bound a multiple of it or the end).
-enum class Form { kTc61, kV2, kG61, kMixed, kFp64 };
+enum class Form { kTc20, kTc61, kV2, kG61, kMixed, kFp64 };
 
 static Form traversal_form(const Session *s) {
+  if (tc20_supported(s)) return Form::kTc20;
   if (tc61_supported(s)) return Form::kTc61;
   if (traverse_v2_supported(s)) return Form::kV2;
   if (g61_supported(s)) return Form::kG61;
@@ -295,13 +287,8 @@ static Form traversal_form(const Session *s) {
 
 static int pattern_granule(const Session *s) {
   switch (traversal_form(s)) {
+    case Form::kTc20:
     case Form::kTc61: return 128;
-    // any range, but mixed 20-state sessions keep to their 128-pattern tiles
-    case Form::kV2:
-      return s->desc.nstates == 20 && s->desc.precision == GEMS_PREC_MIXED &&
-                     s->desc.ncat <= 4 && s->tc_enabled
-                 ? 128
-                 : 1;
     case Form::kG61: return g61_pattern_granule(s);
     default: return 1;
   }
@@ -325,6 +312,10 @@ static int run_ops_range(Session *s, const gems_op *ops, int nops, int p0, int p
   int st = upload_ops(s, ops, nops);
   if (st) return st;
   switch (traversal_form(s)) {
+    case Form::kTc20:
+      if ((st = launch_prep_ops_tc20(s, nops))) return st;
+      if ((st = launch_traverse_tc20(s, nops, p0, p1))) return st;
+      break;
     case Form::kTc61:
       if ((st = launch_prep_ops_tc61(s, nops))) return st;
       if ((st = launch_traverse_tc61(s, nops, p0, p1))) return st;
@@ -385,7 +376,7 @@ static int enqueue_branch_lnl(Session *s, const gems_branch *br, const gems_op *
 static int launch_branch_lnl(Session *s, const gems_branch *br, double *lnl,
                              const gems_op *ops = nullptr, int nops = 0) {
   if (int st = enqueue_branch_lnl(s, br, ops, nops)) return st;
-  if (int st = sync_session(s)) return st;
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
   *lnl = terms_lnl(s);
   return GEMS_OK;
 }
@@ -540,8 +531,6 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
     return fail(e, "cudaHostAlloc jobs");
   if ((e = cudaHostAlloc((void **)&s->h_result, 16 * sizeof(double), 0)) != cudaSuccess)
     return fail(e, "cudaHostAlloc result");
-  s->h_status = reinterpret_cast<int *>(s->h_result + 15);
-  *s->h_status = 0;
   if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(e, "cudaStreamCreate");
   // padded patterns: unknown state, weight 0, zero scale counters
@@ -602,7 +591,8 @@ int gems_session_set_option(gems_session *s, int option, int value) {
       if (value < 1 || value > 64) return GEMS_ERR_BAD_ARG;
       s->newton_share = value;
       return GEMS_OK;
-    case GEMS_OPT_TC20_HALVES:  // accepted: the 20-state mixed form has one schedule
+    case GEMS_OPT_TC20_HALVES:
+      s->tc20_halves = value != 0;
       return GEMS_OK;
     case GEMS_OPT_TC61_ROLES:
       s->tc61_roles = value != 0;
@@ -793,7 +783,8 @@ int gems_traverse(gems_session *s, const gems_op *ops, int nops) {
   GEMS_CUDA(cudaSetDevice(s->desc.device));
   int st = run_ops(s, ops, nops);
   if (st) return st;
-  return sync_session(s);
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  return GEMS_OK;
 }
 
 int gems_session_pattern_granule(gems_session *s, int *granule) {
@@ -817,7 +808,8 @@ int gems_compute_partial(gems_session *s, const gems_op *op, int ptn_lower, int 
   const int p1 = ptn_upper == n ? s->P : ptn_upper;
   int st = run_ops_range(s, op, 1, ptn_lower, p1);
   if (st) return st;
-  return sync_session(s);
+  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  return GEMS_OK;
 }
 
 // every session's own op list (ops[i], nops[i]); sessions must share device, pattern count,
@@ -854,8 +846,7 @@ static int traverse_batch_lists(gems_session *const *ss, int nsess, const gems_o
   if (!tc || nops[0] == 0) {
     for (int i = 0; i < nsess; i++)
       if (int st = run_ops(ss[i], ops[i], nops[i])) return st;
-    for (int i = 0; i < nsess; i++)
-      if (int st = sync_session(ss[i])) return st;
+    for (int i = 0; i < nsess; i++) GEMS_CUDA(cudaStreamSynchronize(ss[i]->stream));
     return GEMS_OK;
   }
   // one op list shared by every session (candidate models on one tree): validated and planned
@@ -905,7 +896,7 @@ int gems_branch_lnl_batch_ops(gems_session *const *ss, int nsess, const gems_op 
   for (int i = 0; i < nsess; i++)
     if (int st = enqueue_branch_lnl(ss[i], &br[i])) return st;
   for (int i = 0; i < nsess; i++) {
-    if (int st = sync_session(ss[i])) return st;
+    GEMS_CUDA(cudaStreamSynchronize(ss[i]->stream));
     lnl[i] = terms_lnl(ss[i]);
   }
   return GEMS_OK;
@@ -955,7 +946,7 @@ int gems_branch_lnl_from_host(gems_session *s, const uint8_t *states, const doub
     set_error("model not set");
     return GEMS_ERR_STATE;
   }
-  const bool ranged = traversal_form(s) == Form::kV2;
+  const bool ranged = traverse_v2_supported(s) && !tc20_supported(s) && !tc61_supported(s);
   if (!ranged || nchunks == 1 || nops == 0) {
     if ((st = gems_upload_tips(s, states))) return st;
     if ((st = gems_upload_patterns(s, ptn_freq, ptn_invar))) return st;

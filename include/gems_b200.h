@@ -98,10 +98,8 @@ int gems_session_sync(gems_session *s);
 int gems_session_info(gems_session *s, gems_session_desc *desc);
 /* the CUDA stream (cudaStream_t) the session launches on, for event timing by the caller */
 int gems_session_stream(gems_session *s, void **stream);
-/* Session options.  GEMS_OPT_TENSOR_CORES (default 1): the mixed-precision 61-state SAFE
- * traversal runs on tcgen05 split-TF32 products; 0 selects the FP32 CUDA-core kernel.  The
- * 20-state one runs in FP32 either way (the option keeps its pattern granule: 128 when set and
- * 1 to 4 categories, else 1).
+/* Session options.  GEMS_OPT_TENSOR_CORES (default 1): the mixed-precision 20-state traversal
+ * runs on tcgen05 split-TF32 products; 0 selects the FP32 CUDA-core kernel.
  * GEMS_OPT_TILED_FP64 (default 1): the FP64 61-state traversal (1 to 8 categories) runs as
  * register-tiled GEMMs over 128-row tiles; 0 selects the per-row kernel (same values, bit for
  * bit). */
@@ -111,8 +109,10 @@ enum { GEMS_OPT_TENSOR_CORES = 1, GEMS_OPT_TILED_FP64 = 2, GEMS_OPT_AUTOTUNE = 3
  * different warps (operand split, MMA issue, epilogue, copies) working on consecutive steps at
  * once, with double-buffered accumulators; 0 selects the form in which every warp runs the
  * parts one after the other.  The values are the same bits either way. */
-/* GEMS_OPT_TC20_HALVES: accepted and without effect (the mixed 20-state traversal has one
- * schedule). */
+/* GEMS_OPT_TC20_HALVES (default 0): the tcgen05 20-state traversal runs two CTAs per SM, each
+ * taking its tile two categories at a time with every internal child copied back from the
+ * slot (no forwarding), instead of one CTA per SM with all categories at once; the values are
+ * the same bits either way. */
 /* GEMS_OPT_NEWTON_SHARE (default 1): the device Newton loop (gems_newton_branch) is one
  * cooperative kernel whose blocks are all resident at once; with value k it takes at most 1/k
  * of the GPU's resident blocks, so that it runs beside other sessions' work instead of waiting
