@@ -281,6 +281,7 @@ int launch_prep_ops_mixed(Session *s, int nops);
 int launch_traverse_mixed(Session *s, int nops, int p0, int p1);
 // theta of a 20- or 61-state branch, and with want_lnl its lnL (as enqueue_terms)
 int enqueue_theta_mixed(Session *s, const gems_branch *br, bool want_lnl, bool store_theta);
+int enqueue_lnl_mixed_batch(Session *const *ss, const gems_branch *br, int n);
 // factored whole-traversal kernels for 4 and 20 states (kernels_traverse.cu)
 bool traverse_v2_supported(const Session *s);
 int launch_prep_ops_v2(Session *s, int nops);
@@ -308,8 +309,9 @@ bool tc61_supported(const Session *s);
 int launch_prep_ops_tc61(Session *s, int nops);
 // p0 a multiple of 128, p1 a multiple of 128 or P
 int launch_traverse_tc61(Session *s, int nops, int p0, int p1);
+// shared_ops: one op list for every session (null: each its own)
 int launch_traverse_tc61_batch(Session *const *ss, int nsess, int nops, int p0, int p1,
-                               bool with_tables);
+                               bool with_tables, const DevOp *shared_ops);
 // FP64 61-state traversal as register-tiled GEMMs, C in {1, 2, 4, 8} (kernels_g61.cu)
 size_t g61_op_doubles(int ncat, int unknown);
 bool g61_supported(const Session *s);

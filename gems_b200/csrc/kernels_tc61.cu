@@ -999,7 +999,7 @@ int launch_prep_ops_tc61(Session *s, int nops) {
 // count, categories and device), on the stream of ss[0]; with_tables: the sessions' op tables
 // are built first, by one launch over every (session, op, side)
 int launch_traverse_tc61_batch(Session *const *ss, int nsess, int nops, int p0, int p1,
-                               bool with_tables) {
+                               bool with_tables, const DevOp *shared_ops) {
   if (nops <= 0 || nsess <= 0 || p1 <= p0) return GEMS_OK;
   Session *s0 = ss[0];
   if (p0 % kTile != 0 || (p1 % kTile != 0 && p1 != s0->P)) {
@@ -1013,7 +1013,7 @@ int launch_traverse_tc61_batch(Session *const *ss, int nsess, int nops, int p0, 
   std::vector<TcJob> jobs(nsess);
   for (int i = 0; i < nsess; i++) {
     jobs[i].c = ss[i]->ctx();
-    jobs[i].ops = ss[i]->d_ops;
+    jobs[i].ops = shared_ops ? shared_ops : ss[i]->d_ops;
     jobs[i].tab = reinterpret_cast<const float *>(ss[i]->d_opmats);
   }
   // host staging (pinned), then one copy; the previous launch that read it has completed
@@ -1057,7 +1057,7 @@ int launch_traverse_tc61_batch(Session *const *ss, int nsess, int nops, int p0, 
 
 int launch_traverse_tc61(Session *s, int nops, int p0, int p1) {
   Session *one[1] = {s};
-  return launch_traverse_tc61_batch(one, 1, nops, p0, p1, false);
+  return launch_traverse_tc61_batch(one, 1, nops, p0, p1, false, nullptr);
 }
 
 }  // namespace gems

@@ -406,6 +406,13 @@ __global__ void k_tips_max(const uint8_t *__restrict__ tips, int P, int nptn, in
   if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
+struct RatePack {
+  double v[2 * kMaxCat];
+};
+__global__ void k_set_rates(double *dst, RatePack r, int n) {
+  if ((int)threadIdx.x < n) dst[threadIdx.x] = r.v[threadIdx.x];
+}
+
 // copies rows of nptn tip bytes (host or device, row stride src_pitch) into the session and
 // checks them on the device: on a bad byte the tips of the session are invalid (traversals are
 // refused) until the next successful load
@@ -709,12 +716,16 @@ int gems_set_rates(gems_session *s, const double *rates, const double *props) {
     if (!(rates[c] >= 0) || !(props[c] >= 0)) return GEMS_ERR_BAD_ARG;
   GEMS_CUDA(cudaSetDevice(s->desc.device));
   // the model block is [eval n][evec n*n][inv_evec n*n][rates C][props C][tip tables]: only the
-  // rates and proportions change (the tip tables depend on inv_evec alone)
-  std::vector<double> rp(rates, rates + C);
-  rp.insert(rp.end(), props, props + C);
-  GEMS_CUDA(cudaMemcpyAsync(s->d_model + n + 2 * (size_t)n * n, rp.data(), rp.size() * sizeof(double),
-                            cudaMemcpyHostToDevice, s->stream));
-  GEMS_CUDA(cudaStreamSynchronize(s->stream));
+  // rates and proportions change (the tip tables depend on inv_evec alone), in stream order (a
+  // kernel parameter: no staging to wait for)
+  RatePack rp{};
+  for (int c = 0; c < C; c++) {
+    rp.v[c] = rates[c];
+    rp.v[C + c] = props[c];
+  }
+  k_set_rates<<<1, 32, 0, s->stream>>>(s->d_model + n + 2 * (size_t)n * n, rp, 2 * C);
+  s->launches++;
+  GEMS_CUDA(cudaGetLastError());
   s->theta_valid = false;
   return GEMS_OK;
 }
@@ -849,30 +860,22 @@ static int traverse_batch_lists(gems_session *const *ss, int nsess, const gems_o
     for (int i = 0; i < nsess; i++) GEMS_CUDA(cudaStreamSynchronize(ss[i]->stream));
     return GEMS_OK;
   }
-  // one op list shared by every session (candidate models on one tree): validated and planned
-  // once, the plan copied to each session
+  // one op list for every session (candidate models on one tree): validated, planned and copied
+  // once, and read by every session's tables and tiles
   bool shared = true;
   for (int i = 1; i < nsess; i++)
-    shared = shared && ops[i] == ops[0] && ss[i]->desc.ntaxa == s0->desc.ntaxa &&
-             ss[i]->nops_max == s0->nops_max;
+    shared = shared && ss[i]->desc.ntaxa == s0->desc.ntaxa && ss[i]->nops_max == s0->nops_max &&
+             (ops[i] == ops[0] || !std::memcmp(ops[i], ops[0], sizeof(gems_op) * nops[0]));
   if (int st = upload_ops(s0, ops[0], nops[0])) return st;
-  for (int i = 1; i < nsess; i++) {
-    Session *s = ss[i];
-    if (!shared) {
-      if (int st = upload_ops(s, ops[i], nops[i])) return st;
-      continue;
-    }
-    GEMS_CUDA(cudaStreamSynchronize(s->stream));  // no kernel still reads its op table
-    std::memcpy(s->h_ops, s0->h_ops, sizeof(DevOp) * nops[0]);
-    s->plan_depth = s0->plan_depth;
-    GEMS_CUDA(cudaMemcpyAsync(s->d_ops, s->h_ops, sizeof(DevOp) * nops[0], cudaMemcpyHostToDevice,
-                              s->stream));
-  }
+  for (int i = 1; i < nsess && !shared; i++)
+    if (int st = upload_ops(ss[i], ops[i], nops[i])) return st;
   // the batched launches (every session's op tables, then the traversal) run on the first
-  // session's stream after every session's op list is on the device
+  // session's stream after every session's earlier work
   for (int i = 1; i < nsess; i++) GEMS_CUDA(cudaStreamSynchronize(ss[i]->stream));
   std::vector<Session *> v(ss, ss + nsess);
-  if (int st = launch_traverse_tc61_batch(v.data(), nsess, nops[0], 0, s0->P, true)) return st;
+  if (int st = launch_traverse_tc61_batch(v.data(), nsess, nops[0], 0, s0->P, true,
+                                          shared ? s0->d_ops : nullptr))
+    return st;
   for (int i = 0; i < nsess; i++) invalidate_theta(ss[i], ops[i], nops[i]);
   return GEMS_OK;
 }
@@ -892,7 +895,20 @@ int gems_branch_lnl_batch_ops(gems_session *const *ss, int nsess, const gems_op 
     if (ss[i])
       if (int st = check_branch(ss[i], &br[i])) return st;
   if (int st = traverse_batch_lists(ss, nsess, ops, nops)) return st;
-  // every session's branch terms enqueued on its own stream first, then the results read
+  // mixed 20- and 61-state sessions: one launch for all, after their streams' work (the traversal
+  // has been waited for); else each on its own stream, then the results read
+  Session *s0 = ss[0];
+  bool lift = nsess > 1 && !theta_in_kernel(s0);
+  for (int i = 1; i < nsess; i++)
+    lift = lift && ss[i]->desc.precision == s0->desc.precision &&
+           ss[i]->desc.scaling == s0->desc.scaling;
+  if (lift) {
+    std::vector<Session *> v(ss, ss + nsess);
+    if (int st = enqueue_lnl_mixed_batch(v.data(), br, nsess)) return st;
+    GEMS_CUDA(cudaStreamSynchronize(s0->stream));
+    for (int i = 0; i < nsess; i++) lnl[i] = terms_lnl(ss[i]);
+    return GEMS_OK;
+  }
   for (int i = 0; i < nsess; i++)
     if (int st = enqueue_branch_lnl(ss[i], &br[i])) return st;
   for (int i = 0; i < nsess; i++) {

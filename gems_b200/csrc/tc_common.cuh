@@ -1,7 +1,7 @@
-// tc_common.cuh -- PTX wrappers shared by the tcgen05 traversal kernels (20 and 61 states):
-// mbarriers with bounded waits, bulk copies, UMMA shared-memory descriptors, tcgen05.mma
-// kind::tf32 (A in shared or tensor memory), commit, fences, lane election, TMEM stores, and
-// the TF32 hi/lo split.
+// tc_common.cuh -- PTX wrappers shared by the tcgen05 traversal kernels (20 and 61 states) and,
+// for its barriers, the Newton kernel: mbarriers with bounded waits, bulk copies, UMMA
+// shared-memory descriptors, tcgen05.mma kind::tf32 (A in shared or tensor memory), commit, fences,
+// lane election, TMEM stores, and the TF32 hi/lo split.
 #pragma once
 
 #include <cstdint>
@@ -80,10 +80,6 @@ __device__ __forceinline__ bool bar_or(bool pred) {
       : "r"((uint32_t)pred), "n"(BAR), "n"(NT)
       : "memory");
   return r != 0;
-}
-template <int BAR, int NT>
-__device__ __forceinline__ void bar_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NT) : "memory");
 }
 // contiguous global -> shared copy completing on an mbarrier (16-byte aligned, size % 16 == 0)
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes,

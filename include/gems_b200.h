@@ -100,8 +100,8 @@ int gems_session_info(gems_session *s, gems_session_desc *desc);
 int gems_session_stream(gems_session *s, void **stream);
 /* Session options.  GEMS_OPT_TENSOR_CORES (default 1): the mixed-precision 20-state traversal
  * runs on tcgen05 split-TF32 products; 0 selects the FP32 CUDA-core kernel.
- * GEMS_OPT_TILED_FP64 (default 1): the FP64 61-state traversal (1 to 8 categories) runs as
- * register-tiled GEMMs over 128-row tiles; 0 selects the per-row kernel (same values, bit for
+ * GEMS_OPT_TILED_FP64 (default 1): the FP64 61-state traversal (1 to 8 categories) runs on the
+ * FP64 tensor instructions (SAFE) or as register-tiled GEMMs (NORM); 0 selects the per-row kernel (same values, bit for
  * bit). */
 enum { GEMS_OPT_TENSOR_CORES = 1, GEMS_OPT_TILED_FP64 = 2, GEMS_OPT_AUTOTUNE = 3,
        GEMS_OPT_NEWTON_SHARE = 4, GEMS_OPT_TC20_HALVES = 5, GEMS_OPT_TC61_ROLES = 6 };
