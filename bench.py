@@ -468,7 +468,7 @@ def protein_comparison(args, local, peaks):
         ms, lnl, kms, _ = time_lnl(gt, max(args.steps, 5), 3, stream, None, lnl_buf)
         b_ii, b_ti, b_tt = update_bytes(8 if prec == "fp64" else 4, n, C)
         alg = aln.npat * (kinds[0] * b_ii + kinds[1] * b_ti + kinds[2] * b_tt)
-        unit, pk = {"fp64": ("fp64 FMA", peaks["fp64_tflops"]),
+        unit, pk = {"fp64": ("fp64 mma.sync (the rate of fp64 FMA)", peaks["fp64_tflops"]),
                     "mixed_tcgen05": ("tcgen05 TF32 (3 products issued per credited one)",
                                       peaks["tf32_tflops"]),
                     "mixed_cuda_cores": ("fp32 FMA", peaks["fp32_tflops"])}[name]
@@ -479,8 +479,8 @@ def protein_comparison(args, local, peaks):
                                   "peak": hbm_peak, "peak_source": peak_src, "unit": "GB/s",
                                   "frac": alg / (kms * 1e-3) / 1e9 / hbm_peak,
                                   "algorithmic_bytes_per_launch": alg,
-                                  "traffic": read_traffic("traverse_mixed_protein128.md")
-                                  if name == "mixed_tcgen05" else None},
+                                  "traffic": read_traffic(f"traverse_{prec}_protein128.md")
+                                  if tc else None},
                      "compute": {"unit_used": unit, "achieved_tflops": flops / (kms * 1e-3) / 1e12,
                                  "peak_tflops": pk, "frac": flops / (kms * 1e-3) / 1e12 / pk,
                                  "algorithmic_flops_per_launch": flops}}
