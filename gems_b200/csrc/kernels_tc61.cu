@@ -70,19 +70,26 @@ constexpr uint32_t kTipBytes61 = kTipRows61 * kTipRow61 * 4;  // 16,864 bytes
 
 // The op tables of a job's op k and side (blockIdx.x, blockIdx.y; job blockIdx.z of `jobs`, or
 // `one` when jobs is null).  P_c(t) = evec . diag(exp(eval * rate_c * t)) . inv_evec in FP64,
-// clamped at 0, then split into TF32 hi and lo images.  Register-tiled: a thread owns target
-// states 4xq..4xq+3 by the source-state quads jo and jo + 8 (4 x 8 outputs; float4s of the
-// image rows it writes), so each term of the sum costs 13 shared-memory reads for 32 FMAs; the
-// sum over i runs in index order with the same fma(evec * exp, inv_evec, acc) steps as a scalar
-// loop.  Shared memory: exp terms [C][n]; evec as [64][n] (rows 61..63 zero); inv_evec as
-// [n][4 e][16 j] = inv_evec[i][4j + e] (columns 61..63 zero), so that the 8 lanes of a row quad
-// read 8 consecutive doubles.  A tip side's unknown-state row sums add the quads j and j + 8 in
-// the thread, then the 8 lanes of the row quad by a fixed shuffle tree: the same bits in every
-// launch.
-// two halves of 128 threads (16 row quads x 8 pairs of column quads) take alternate categories
+// clamped at 0, then split into TF32 hi and lo images.  A 61 x 61 x 61 product per category: the
+// FP64 mma (m8n8k4), a warp 16 target states by all 64 source states (2 x 8 tiles), four warps a
+// category, two categories at a time.  The mma adds in index order, so the tables have the bits
+// of a loop of fma(evec * exp, inv_evec, acc).  Shared memory: exp terms [C][64], evec and
+// inv_evec in fragment order (zero padded), read without conflicts: 19 reads of 32 lanes for 16
+// mma, whose 64 cycles bound the kernel.  Column n of N tile (h, p) is source state
+// 4 (n / 2 + 4h) + 2p + n % 2, so that a lane ends with whole quads of a row of an image; row g of
+// M tile m is target state 8m + g of the warp's 16 for an image (eight lanes write 128
+// consecutive bytes) and 2g + m for a tip table, whose rows are source states.  A tip side's
+// unknown-state row sums add by a fixed tree: quads j and j + 8, then over j.
+// Measured: 32 codon +G4 models of 198 ops, an evaluation of 12.06 ms with a thread per 4 x 8
+// outputs on FMA (13 shared-memory reads for 32 of them), 11.78 ms so.
 constexpr int kPrepThreads = 256;
 __host__ __device__ constexpr size_t prep61_smem_doubles(int C) {
-  return (size_t)C * kN + (size_t)kNP * kN + (size_t)kN * kNP;
+  return (size_t)C * kNP + 2 * (size_t)kNP * kNP;
+}
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 __global__ void __launch_bounds__(kPrepThreads, 2)
     k_prep_ops_tc61(const __grid_constant__ TcJob one, const TcJob *__restrict__ jobs,
@@ -93,100 +100,90 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
   const int k = blockIdx.x, side = blockIdx.y;
   const DevOp op = job.ops[k];
   const double len = side ? op.r_len : op.l_len;
+  const bool tip = (side ? op.r_kind : op.l_kind) == GEMS_CHILD_TIP;
   const int C = c.C, n = kN;
-  double *ev = ex + C * n, *iv = ev + kNP * n;
-  for (int idx = threadIdx.x; idx < C * n; idx += blockDim.x) {
-    const int cc = idx / n, i = idx - cc * n;
-    ex[idx] = exp(c.eval[i] * (c.rates[cc] * len));
+  double *fa = ex + C * kNP, *fb = fa + kNP * kNP;
+  for (int idx = threadIdx.x; idx < C * kNP; idx += blockDim.x) {
+    const int cc = idx / kNP, i = idx % kNP;
+    ex[idx] = i < n ? exp(c.eval[i] * (c.rates[cc] * len)) : 0.0;
   }
-  for (int idx = threadIdx.x; idx < kNP * n; idx += blockDim.x) {
-    const int x = idx / n;
-    ev[idx] = x < n ? c.evec[idx] : 0.0;
-    const int i = idx / kNP, r = idx - i * kNP, e = r >> 4, j = r & 15, y = 4 * j + e;
-    iv[idx] = y < n ? c.inv_evec[i * n + y] : 0.0;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < kNP * kNP; idx += kPrepThreads) {
+    const int q = idx >> 5;  // fragment: A [warp][M tile][K step], B [K step][N tile]
+    const int xa = 16 * (q >> 5) + (tip ? 2 * g + ((q >> 4) & 1) : 8 * ((q >> 4) & 1) + g);
+    const int ia = 4 * (q & 15) + t;
+    fa[idx] = xa < n && ia < n ? c.evec[xa * n + ia] : 0.0;
+    const int ib = 4 * (q >> 3) + t, y = 4 * ((g >> 1) + 4 * ((q >> 1) & 3)) + 2 * (q & 1) + (g & 1);
+    fb[idx] = ib < n && y < n ? c.inv_evec[ib * n + y] : 0.0;
   }
   __syncthreads();
   // the job's own table, written here and read by its traversal
   float *img = const_cast<float *>(job.tab) + (size_t)k * stride_f + (size_t)side * C * (kBSide / 4);
   const int per = kBImg / 4;  // floats of one image
-  // thread: row quad xq (rows 4xq..4xq+3) and the column quads jo and jo + 8, in the half of
-  // the block that takes categories sub, sub + 2, ...
-  const int lt = threadIdx.x & 127, sub = threadIdx.x >> 7;
-  const int jo = lt & 7, xq = lt >> 3;
-  const bool tip = (side ? op.r_kind : op.l_kind) == GEMS_CHILD_TIP;
+  const int w = (threadIdx.x >> 5) & 3, sub = threadIdx.x >> 7;
+  const double *wa = fa + w * 2 * 16 * 32 + lane, *wb = fb + lane;
   for (int cc = sub; cc < C; cc += 2) {
-    double acc[4][2][4];  // [row][column quad jo, jo + 8][column in quad]
+    double acc[2][8][2];  // [M tile][N tile][column]
 #pragma unroll
-    for (int r = 0; r < 4; r++)
+    for (int m = 0; m < 2; m++)
 #pragma unroll
-      for (int h = 0; h < 2; h++)
+      for (int q = 0; q < 8; q++) acc[m][q][0] = acc[m][q][1] = 0.0;
+    __syncwarp();
+#pragma unroll 2
+    for (int s = 0; s < 16; s++) {
+      const double xi = ex[cc * kNP + 4 * s + t];
+      const double a0 = wa[s * 32] * xi, a1 = wa[(16 + s) * 32] * xi;
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[r][h][e] = 0.0;
-    const double *exc = ex + cc * n;
-    for (int i = 0; i < n; i++) {
-      const double xi = exc[i];
-      double a[4], b[2][4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) a[r] = ev[(4 * xq + r) * n + i] * xi;
-#pragma unroll
-      for (int h = 0; h < 2; h++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) b[h][e] = iv[i * kNP + e * 16 + jo + 8 * h];
-#pragma unroll
-      for (int r = 0; r < 4; r++)
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) acc[r][h][e] = fma(a[r], b[h][e], acc[r][h][e]);
+      for (int q = 0; q < 8; q++) {
+        const double b = wb[(s * 8 + q) * 32];
+        dmma(acc[0][q], a0, b);
+        dmma(acc[1][q], a1, b);
+      }
     }
     if (tip) {
       // tip table: row s = column s of P_c (target states x consecutive), then the row sums
-      float *tt = img + (size_t)cc * 2 * per;
-      double rs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+      float *tt = img + (size_t)cc * 2 * per + 16 * w + 2 * g;
+      double rs[4][2];
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int j = jo + 8 * h;
+      for (int h = 0; h < 4; h++) {
+        rs[h][0] = rs[h][1] = 0.0;
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          const int y = 4 * j + e;
-          float v[4];
+          const int y = 4 * (t + 4 * h) + e;
+          double v[2];
 #pragma unroll
-          for (int r = 0; r < 4; r++) {
-            const int x = 4 * xq + r;
-            const double a = (x < n && y < n) ? fmax(acc[r][h][e], 0.0) : 0.0;
-            rs[h][r] += a;
-            v[r] = (float)a;
+          for (int m = 0; m < 2; m++) {
+            v[m] = 16 * w + 2 * g + m < n && y < n ? fmax(acc[m][2 * h + (e >> 1)][e & 1], 0.0) : 0.0;
+            rs[h][m] += v[m];
           }
           if (y < n)
-            *reinterpret_cast<float4 *>(tt + (size_t)y * kTipRow61 + 4 * xq) =
-                make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float2 *>(tt + (size_t)y * kTipRow61) =
+                make_float2((float)v[0], (float)v[1]);
         }
       }
-      // the sums of the 16 column quads by a fixed tree: quads j and j + 8 first (in this
-      // thread), then across the 8 lanes of the row quad
-      double t4[4];
+      double sum[2];
 #pragma unroll
-      for (int r = 0; r < 4; r++) t4[r] = rs[0][r] + rs[1][r];
-#pragma unroll
-      for (int o = 4; o >= 1; o >>= 1)
-#pragma unroll
-        for (int r = 0; r < 4; r++) t4[r] += __shfl_xor_sync(0xffffffffu, t4[r], o);
-      if (jo == 0)
-        *reinterpret_cast<float4 *>(tt + (size_t)n * kTipRow61 + 4 * xq) =
-            make_float4((float)t4[0], (float)t4[1], (float)t4[2], (float)t4[3]);
+      for (int m = 0; m < 2; m++) {
+        sum[m] = (rs[0][m] + rs[2][m]) + (rs[1][m] + rs[3][m]);
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 2);
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
+      }
+      if (t == 0)
+        *reinterpret_cast<float2 *>(tt + (size_t)n * kTipRow61) =
+            make_float2((float)sum[0], (float)sum[1]);
       continue;
     }
     // image element (row x, K index y) at chunk y / 4, row x, lane y % 4
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int x = 4 * xq + r;
+    for (int h = 0; h < 4; h++)
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int j = jo + 8 * h;
+      for (int m = 0; m < 2; m++) {
+        const int x = 16 * w + 8 * m + g, j = t + 4 * h;
         float v[4];
 #pragma unroll
         for (int e = 0; e < 4; e++)
-          v[e] = (x < n && 4 * j + e < n) ? (float)fmax(acc[r][h][e], 0.0) : 0.f;
+          v[e] = x < n && 4 * j + e < n ? (float)fmax(acc[m][2 * h + (e >> 1)][e & 1], 0.0) : 0.f;
         const float4 hi = make_float4(tf32_rna(v[0]), tf32_rna(v[1]), tf32_rna(v[2]), tf32_rna(v[3]));
         const float4 lo = make_float4(tf32_rna(v[0] - hi.x), tf32_rna(v[1] - hi.y),
                                       tf32_rna(v[2] - hi.z), tf32_rna(v[3] - hi.w));
@@ -194,7 +191,6 @@ __global__ void __launch_bounds__(kPrepThreads, 2)
         *reinterpret_cast<float4 *>(img + o) = hi;
         *reinterpret_cast<float4 *>(img + o + per) = lo;
       }
-    }
   }
 }
 
