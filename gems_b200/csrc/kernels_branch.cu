@@ -699,6 +699,24 @@ __device__ __forceinline__ void send_pair(uint32_t dst, uint32_t bar, double a, 
       "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(bar)
       : "memory");
 }
+// Bounded wait for what the blocks of the cluster sent, false when it has not all come in time.
+// The senders are other blocks: the acquire is at cluster scope (tc::mbar_wait's, for copies and
+// MMAs of the block itself, is at the block's).
+__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (clock64() - t0 > tc::kWaitCycles) return false;
+  }
+}
 
 struct NewtonArgs {
   gems_branch br;
@@ -850,7 +868,7 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
     if (lane < CS)
       send_pair(cluster_addr(s_recv + (set * kMaxCluster * kWarps + rank * kWarps + warp) * 16, lane),
                 cluster_addr(bar, lane), v0, v1);
-    bool ok = tc::mbar_wait(bar, use);
+    bool ok = cluster_wait(bar, use);
     v0 = v1 = 0.0;
     if (ok)
       for (int i = lane; i < CS * kWarps; i += 32) {
