@@ -16,6 +16,7 @@ static thread_local std::string g_err;
 void set_error(const std::string &msg) { g_err = msg; }
 
 int cuda_status(cudaError_t e, const char *what) {
+  cudaGetLastError();  // reported here: not again by the next call that asks for the last error
   g_err = std::string(what) + ": " + cudaGetErrorString(e);
   if (e == cudaErrorMemoryAllocation) return GEMS_ERR_OOM;
   return GEMS_ERR_CUDA;

@@ -1,0 +1,86 @@
+// Host code of the library on a CUDA runtime without a device (fake_cudart.cpp): error paths,
+// launch shapes and choices by timing that no run on a GPU can bring about on purpose.
+// usage: host_paths CASE (none: lists them); prints OK or the expectation that failed.
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+#include "fake_cudart.h"
+#include "gems_b200.h"
+
+namespace {
+
+#define EXPECT(cond)                                            \
+  do {                                                          \
+    if (!(cond)) {                                              \
+      std::printf("line %d: expected %s\n", __LINE__, #cond);   \
+      std::exit(1);                                             \
+    }                                                           \
+  } while (0)
+
+gems_session *session(int nstates, int ncat, int nptn, int precision, int scaling,
+                      int ntaxa = 8) {
+  gems_session_desc d{ntaxa, nptn, nstates, ncat, ntaxa, precision, scaling, 0};
+  gems_session *s = nullptr;
+  EXPECT(gems_session_create(&d, &s) == GEMS_OK);
+  std::vector<uint8_t> tips((size_t)ntaxa * nptn, 1);
+  EXPECT(gems_upload_tips(s, tips.data()) == GEMS_OK);
+  std::vector<double> freq(nptn, 1.0), eval(nstates, -1.0), ev((size_t)nstates * nstates, 0.5);
+  EXPECT(gems_upload_patterns(s, freq.data(), nullptr) == GEMS_OK);
+  std::vector<double> r(ncat, 1.0), p(ncat, 1.0 / ncat);
+  EXPECT(gems_set_model(s, eval.data(), ev.data(), ev.data(), r.data(), p.data()) == GEMS_OK);
+  return s;
+}
+
+// slot k from tips: `n` updates
+std::vector<gems_op> updates(int n) {
+  std::vector<gems_op> ops;
+  for (int k = 0; k < n; k++)
+    ops.push_back(k == 0 ? gems_op{0, GEMS_CHILD_TIP, 0, GEMS_CHILD_TIP, 1, 0, 0.1, 0.1}
+                         : gems_op{k, GEMS_CHILD_PARTIAL, k - 1, GEMS_CHILD_TIP, k + 1, 0, 0.1, 0.1});
+  return ops;
+}
+const gems_branch kBranch{2, GEMS_CHILD_TIP, 5, 0, 0.1}, kOther{1, GEMS_CHILD_TIP, 6, 0, 0.1};
+
+int count(const char *kernel) {
+  int n = 0;
+  for (const fake::Launch &l : fake::launches) n += l.kernel.find(kernel) != std::string::npos;
+  return n;
+}
+
+std::map<std::string, void (*)()> &cases() {
+  static std::map<std::string, void (*)()> m;
+  return m;
+}
+#define CASE(name)                                                   \
+  void name();                                                       \
+  const bool name##_listed = (cases()[#name] = &name, true);         \
+  void name()
+
+// ---- an error that a call returned is not returned again by the next one --------------------
+CASE(error_once) {
+  gems_session *s = session(20, 4, 300, GEMS_PREC_FP64, GEMS_SCALE_SAFE);
+  const std::vector<gems_op> ops = updates(3);
+  double a, b;
+  fake::fail_kernel = "k_terms";
+  EXPECT(gems_branch_derv(s, ops.data(), 3, &kBranch, 1, &a, &b, nullptr) == GEMS_ERR_CUDA);
+  fake::fail_kernel = "";
+  EXPECT(gems_branch_derv(s, ops.data(), 3, &kBranch, 1, &a, &b, nullptr) == GEMS_OK);
+  EXPECT(gems_session_destroy(s) == GEMS_OK);
+}
+
+}  // namespace
+
+int main(int argc, char **argv) {
+  if (argc == 1) {
+    for (const auto &c : cases()) std::printf("%s\n", c.first.c_str());
+    return 0;
+  }
+  const auto it = cases().find(argv[1]);
+  if (it == cases().end()) return 2;
+  it->second();
+  std::printf("OK\n");
+  return 0;
+}
