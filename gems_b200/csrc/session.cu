@@ -358,6 +358,24 @@ static int run_branch_ops(Session *s, const gems_op *ops, int nops, int *left) {
   return GEMS_OK;
 }
 
+static void theta_of(Session *s, const gems_branch *br) {
+  s->theta_valid = true;
+  s->theta_branch = *br;
+}
+
+// The node updates and, for sessions whose theta has its own launch, theta of a branch call that
+// forms theta anew.  From here on the session has no theta until the launch that writes it has
+// been made (theta_of): a call that fails between leaves none that a later call would read.
+static int start_theta(Session *s, const gems_op *ops, int nops, const gems_branch *br,
+                       int *left) {
+  if (int st = run_branch_ops(s, ops, nops, left)) return st;
+  s->theta_valid = false;
+  if (theta_in_kernel(s)) return GEMS_OK;
+  if (int st = enqueue_theta_mixed(s, br, false, true)) return st;
+  theta_of(s, br);
+  return GEMS_OK;
+}
+
 static void copy_pattern_lh(Session *s, double *pattern_lh, double lnl_raw_finite) {
   (void)lnl_raw_finite;
   if (!pattern_lh) return;
@@ -1045,16 +1063,14 @@ int gems_branch_derv(gems_session *s, const gems_op *ops, int nops, const gems_b
   int st = check_branch(s, br);
   if (st) return st;
   if (compute_theta) {
-    if ((st = run_branch_ops(s, ops, nops, &left))) return st;
-    if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
-    s->theta_valid = true;
-    s->theta_branch = *br;
+    if ((st = start_theta(s, ops, nops, br, &left))) return st;
   } else if (!s->theta_valid) {
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
   const bool form = compute_theta && theta_in_kernel(s);
   if ((st = launch_derv(s, form ? br : nullptr, br->length, df, ddf, ops, left))) return st;
+  if (compute_theta) theta_of(s, br);
   if (df_frac) {
     GEMS_CUDA(cudaMemcpyAsync(df_frac, s->d_df_frac, sizeof(double) * s->desc.nptn,
                               cudaMemcpyDeviceToHost, s->stream));
@@ -1086,16 +1102,17 @@ int gems_newton_branch_async(gems_session *s, const gems_op *ops, int nops,
   int st = check_branch(s, br);
   if (st) return st;
   if (compute_theta) {
-    if ((st = run_branch_ops(s, ops, nops, &left))) return st;
-    if (!theta_in_kernel(s) && (st = enqueue_theta_mixed(s, br, false, true))) return st;
-    s->theta_valid = true;
-    s->theta_branch = *br;
+    if ((st = start_theta(s, ops, nops, br, &left))) return st;
   } else if (!s->theta_valid) {
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
-  return launch_newton_async(s, compute_theta && theta_in_kernel(s) ? br : nullptr, br->length,
-                             min_len, max_len, xacc, max_steps, ops, left);
+  const bool form = compute_theta && theta_in_kernel(s);
+  if ((st = launch_newton_async(s, form ? br : nullptr, br->length, min_len, max_len, xacc,
+                                max_steps, ops, left)))
+    return st;
+  if (compute_theta) theta_of(s, br);
+  return GEMS_OK;
 }
 
 int gems_newton_branch_wait(gems_session *s, double *opt_len, int *nevals) {

@@ -71,6 +71,39 @@ CASE(error_once) {
   EXPECT(gems_session_destroy(s) == GEMS_OK);
 }
 
+// ---- a launch that forms theta and fails leaves no theta that a later call would read --------
+void theta_after_failure(int nstates, int ncat, int precision, const char *kernel) {
+  gems_session *s = session(nstates, ncat, 300, precision, GEMS_SCALE_SAFE);
+  const std::vector<gems_op> ops = updates(3);
+  double a, b;
+  int n;
+  for (int newton = 0; newton < 2; newton++) {
+    auto form = [&](const gems_branch &br) {
+      return newton ? gems_newton_branch(s, ops.data(), 3, &br, 1, 1e-6, 10.0, 1e-6, 5, &a, &n)
+                    : gems_branch_derv(s, ops.data(), 3, &br, 1, &a, &b, nullptr);
+    };
+    EXPECT(form(kBranch) == GEMS_OK);
+    EXPECT(gems_lnl_from_buffer(s, 0.1, &a, nullptr) == GEMS_OK);
+    fake::fail_kernel = kernel[0] ? kernel : newton ? "k_newton" : "k_terms";
+    EXPECT(form(kOther) == GEMS_ERR_CUDA);
+    fake::fail_kernel = "";
+    EXPECT(gems_lnl_from_buffer(s, 0.1, &a, nullptr) == GEMS_ERR_STATE);
+    EXPECT(gems_branch_derv(s, nullptr, 0, &kBranch, 0, &a, &b, nullptr) == GEMS_ERR_STATE);
+    EXPECT(gems_newton_branch(s, nullptr, 0, &kBranch, 0, 1e-6, 10.0, 1e-6, 5, &a, &n) ==
+           GEMS_ERR_STATE);
+    EXPECT(gems_get_theta(s, nullptr, nullptr) == GEMS_ERR_STATE);
+    EXPECT(form(kOther) == GEMS_OK);
+    EXPECT(gems_branch_derv(s, nullptr, 0, &kOther, 0, &a, &b, nullptr) == GEMS_OK);
+  }
+  EXPECT(gems_session_destroy(s) == GEMS_OK);
+}
+CASE(theta_4_fp64) { theta_after_failure(4, 4, GEMS_PREC_FP64, ""); }
+CASE(theta_4_fp64_one_category) { theta_after_failure(4, 1, GEMS_PREC_FP64, ""); }
+CASE(theta_4_mixed) { theta_after_failure(4, 4, GEMS_PREC_MIXED, ""); }
+CASE(theta_20_fp64) { theta_after_failure(20, 4, GEMS_PREC_FP64, ""); }
+CASE(theta_61_fp64) { theta_after_failure(61, 4, GEMS_PREC_FP64, ""); }
+CASE(theta_20_mixed) { theta_after_failure(20, 4, GEMS_PREC_MIXED, "k_theta_mixed"); }
+
 }  // namespace
 
 int main(int argc, char **argv) {
