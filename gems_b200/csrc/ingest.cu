@@ -392,19 +392,30 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
   return GEMS_OK;
 }
 
-// Writes one byte of every page of a destination that a copy will fill.  A caller's fresh array
-// has no pages yet, and a device copy into it faults them in one by one (43 MB: 10 ms instead of
-// 2.5); a few threads take the faults side by side.
+// Makes the pages of a destination that a copy will fill.  A caller's fresh array has none yet,
+// and a device copy into it faults them in one by one (43 MB: 10 ms instead of 2.5); a few threads
+// take the faults side by side, by a write access that leaves every byte as it is.  Only pageable host memory: pinned memory has its pages, and an address
+// the host cannot write to is for the copy to refuse.
 static void touch_pages(uint8_t *p, size_t n) {
   constexpr size_t kPage = 4096, kLeast = 4u << 20;
   if (n < kLeast) return;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
+    cudaGetLastError();
+    return;
+  }
   const size_t per = 2u << 20;
   const int most = (int)std::min<size_t>(8, std::thread::hardware_concurrency());
   const int nt = (int)std::min<size_t>((size_t)std::max(1, most), n / per);
   auto touch = [p, n, nt](int t) {
     const size_t a = n / nt * t, b = t + 1 == nt ? n : n / nt * (t + 1);
-    for (size_t i = a; i < b; i += kPage) *(volatile uint8_t *)(p + i) = 0;
-    *(volatile uint8_t *)(p + b - 1) = 0;
+    auto page_of = [p](size_t i) {
+      uint8_t v = 0;  // zero for zero, else nothing: a write access either way
+      __atomic_compare_exchange_n(p + i, &v, (uint8_t)0, false, __ATOMIC_RELAXED,
+                                  __ATOMIC_RELAXED);
+    };
+    for (size_t i = a; i < b; i += kPage) page_of(i);
+    page_of(b - 1);
   };
   std::vector<std::thread> ts;
   int t = 1;

@@ -1,6 +1,6 @@
 // A CUDA runtime without a device: what the library's host code calls, on host memory.  "Device"
-// memory is host memory (zeroed), copies are memcpy, kernels do nothing but are recorded by name
-// with their grid and block, and any call or launch can be made to fail.  A virtual clock gives
+// memory is host memory (zeroed), copies are memcpy, kernels do nothing (but what a test does for
+// them) and are recorded by name with their grid and block, and any call or launch can be made to fail.  A virtual clock gives
 // kernels and first uses a duration, for code that decides by timing.
 #include "fake_cudart.h"
 
@@ -16,6 +16,7 @@ std::vector<Launch> launches;
 std::string fail_kernel, fail_call;
 size_t allocated = 0;
 std::set<const void *> device_only;
+std::function<void(const std::string &, void **)> on_launch;
 std::function<double(const std::string &, const Launch &)> kernel_ms;
 std::function<double(const std::string &)> first_use_ms;
 }  // namespace fake
@@ -38,13 +39,14 @@ cudaError_t check(const char *call) {
 void use(const void *fn) {
   if (g_used.insert(fn).second && fake::first_use_ms) g_host += fake::first_use_ms(g_names[fn]);
 }
-cudaError_t launch(const void *fn, dim3 grid, dim3 block) {
+cudaError_t launch(const void *fn, dim3 grid, dim3 block, void **args) {
   const std::string &name = g_names[fn];
   if (!fake::fail_kernel.empty() && name.find(fake::fail_kernel) != std::string::npos)
     return g_last = cudaErrorCooperativeLaunchTooLarge;
   use(fn);
   fake::Launch l{name, (int)grid.x, (int)grid.y, (int)block.x};
   fake::launches.push_back(l);
+  if (fake::on_launch) fake::on_launch(name, args);
   g_stream = (g_stream > g_host ? g_stream : g_host) +
              (fake::kernel_ms ? fake::kernel_ms(name, l) : 0.01);
   return cudaSuccess;
@@ -84,16 +86,16 @@ cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem, vo
   *static_cast<cudaStream_t *>(stream) = g_config.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *fn, dim3 grid, dim3 block, void **, size_t,
+cudaError_t cudaLaunchKernel(const void *fn, dim3 grid, dim3 block, void **args, size_t,
                              cudaStream_t) {
-  return launch(fn, grid, block);
+  return launch(fn, grid, block, args);
 }
-cudaError_t cudaLaunchCooperativeKernel(const void *fn, dim3 grid, dim3 block, void **, size_t,
+cudaError_t cudaLaunchCooperativeKernel(const void *fn, dim3 grid, dim3 block, void **args, size_t,
                                         cudaStream_t) {
-  return launch(fn, grid, block);
+  return launch(fn, grid, block, args);
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fn, void **) {
-  return launch(fn, c->gridDim, c->blockDim);
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fn, void **args) {
+  return launch(fn, c->gridDim, c->blockDim, args);
 }
 cudaError_t cudaMalloc(void **p, size_t n) {
   if (cudaError_t e = check("cudaMalloc")) return e;

@@ -17,6 +17,8 @@ extern std::vector<Launch> launches;
 extern std::string fail_kernel, fail_call;
 extern size_t allocated;                   // bytes of device memory held
 extern std::set<const void *> device_only;  // addresses the runtime takes for device memory
+// called for each launch with the kernel's arguments
+extern std::function<void(const std::string &, void **)> on_launch;
 // duration of a launch, and of what the host does when a kernel is first used
 extern std::function<double(const std::string &, const Launch &)> kernel_ms;
 extern std::function<double(const std::string &)> first_use_ms;

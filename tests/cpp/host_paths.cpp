@@ -1,6 +1,8 @@
 // Host code of the library on a CUDA runtime without a device (fake_cudart.cpp): error paths,
 // launch shapes and choices by timing that no run on a GPU can bring about on purpose.
 // usage: host_paths CASE (none: lists them); prints OK or the expectation that failed.
+#include <sys/mman.h>
+
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -103,6 +105,39 @@ CASE(theta_4_mixed) { theta_after_failure(4, 4, GEMS_PREC_MIXED, ""); }
 CASE(theta_20_fp64) { theta_after_failure(20, 4, GEMS_PREC_FP64, ""); }
 CASE(theta_61_fp64) { theta_after_failure(61, 4, GEMS_PREC_FP64, ""); }
 CASE(theta_20_mixed) { theta_after_failure(20, 4, GEMS_PREC_MIXED, "k_theta_mixed"); }
+
+// ---- an ingest's results: a copy that fails leaves the caller's array as it was, and an address
+// that the host cannot write to is an error of the copy -------------------------------------------
+gems_ingest *ingest(int ntaxa, long long npat) {
+  fake::on_launch = [npat](const std::string &name, void **args) {
+    if (name.find("k_scan_sums") != std::string::npos) **static_cast<long long **>(args[2]) = npat;
+  };
+  std::vector<uint8_t> codes((size_t)ntaxa * npat);
+  gems_ingest *g = nullptr;
+  long long n = 0;
+  EXPECT(gems_ingest_create(0, ntaxa, npat, 4, codes.data(), 1, &g, &n) == GEMS_OK && n == npat);
+  return g;
+}
+CASE(ingest_failed_copy) {
+  gems_ingest *g = ingest(64, 200000);
+  std::vector<uint8_t> out((size_t)64 * 200000, 0xAB);
+  fake::fail_call = "cudaMemcpy";
+  EXPECT(gems_ingest_read(g, out.data(), nullptr, nullptr, nullptr) == GEMS_ERR_CUDA);
+  fake::fail_call = "";
+  for (uint8_t b : out) EXPECT(b == 0xAB);
+  EXPECT(gems_ingest_read(g, out.data(), nullptr, nullptr, nullptr) == GEMS_OK);
+  for (uint8_t b : out) EXPECT(b == 0);
+  gems_ingest_destroy(g);
+}
+CASE(ingest_device_address) {
+  gems_ingest *g = ingest(64, 200000);
+  void *p = mmap(nullptr, (size_t)64 * 200000, PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  EXPECT(p != MAP_FAILED);
+  fake::device_only.insert(p);
+  EXPECT(gems_ingest_read(g, static_cast<uint8_t *>(p), nullptr, nullptr, nullptr) ==
+         GEMS_ERR_CUDA);
+  gems_ingest_destroy(g);
+}
 
 }  // namespace
 
