@@ -262,6 +262,8 @@ bool small_ops(const Session *s, int nops);
 int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length,
                   const gems_op *ops, int nops);
 double terms_lnl(const Session *s);
+// theta of a branch alone, for the launches after it
+int enqueue_theta(Session *s, const gems_branch *br);
 int launch_derv(Session *s, const gems_branch *br, double length, double *df, double *ddf,
                 const gems_op *ops, int nops);
 int launch_from_buffer(Session *s, double length, double *lnl);

@@ -507,7 +507,8 @@ constexpr int kThreadsT = 256;
 constexpr int ctas_t(int e2) { return e2 <= 2 ? 3 : (e2 <= 5 ? 2 : 1); }
 
 // One evaluation at length t: flags kStore (theta and scale_all kept), kLnl (pattern_lh; out =
-// lnL, lnL with non-finite patterns clamped) or kDerv (df_frac, ddf_term; out = df, ddf).
+// lnL, lnL with non-finite patterns clamped) or kDerv (df_frac, ddf_term; out = df, ddf); kStore
+// alone: theta only.
 template <int SRC, bool SAFE, int E2>
 __global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
     k_terms(DevCtx c, gems_branch br, double t, int L, int flags, unsigned int *ticket,
@@ -551,6 +552,7 @@ __global__ void __launch_bounds__(kThreadsT, ctas_t(E2))
           store_theta<E2>(c, L, l, pu[u], th[u]);
           if (l == 0) c.scale_all[pu[u]] = (double)ms[u] * thr;
         }
+      if (flags == kStore) continue;
     }
     const double lh = lanes_sum2(dot<E2>(th[0], tab, L, l), dot<E2>(th[1], tab, L, l), L, l);
     double d1 = 0.0, d2 = 0.0;
@@ -1024,8 +1026,8 @@ static SmallOps small_list(const gems_op *ops, int nops) {
 
 // br: theta from the branch's partials; null: theta as stored.  The two results are in
 // s->h_result once the stream has completed.
-int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length,
-                  const gems_op *ops, int nops) {
+static int launch_terms(Session *s, const gems_branch *br, int flags, int id, double length,
+                        const gems_op *ops, int nops) {
   DevCtx c = s->ctx();
   SmallOps o = small_list(ops, nops);
   Split sp = split_of(s->block, s->desc.ncat);
@@ -1034,18 +1036,26 @@ int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, doubl
   const int grid = (int)std::min<long>(148 * ctas_t(sp.E2), (s->P + per - 1) / per);
   gems_branch b{};
   if (br) b = *br;
-  int flags = (store ? kStore : 0) | (lnl ? kLnl : kDerv);
-  const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * (lnl ? 1 : 3) +
+  const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * (flags & kDerv ? 3 : 1) +
                                         small_doubles(nops, s->desc.ncat, mixed_of(s)));
   unsigned int *ticket = s->d_bar;
   double *out = s->h_result;
   void *args[] = {&c, &b, &length, &sp.L, &flags, &ticket, &out, &o};
-  const int id = lnl ? (br ? 1 : 4) : 3;
   cudaEvent_t ev0;
   if (int st = prof_begin(s, id, &ev0)) return st;
   GEMS_CUDA(cudaLaunchKernel(f.terms, dim3(grid), dim3(kThreadsT), args, smem, s->stream));
   s->launches++;
   return prof_end(s, id, ev0);
+}
+
+int enqueue_terms(Session *s, const gems_branch *br, bool store, bool lnl, double length,
+                  const gems_op *ops, int nops) {
+  return launch_terms(s, br, (store ? kStore : 0) | (lnl ? kLnl : kDerv), lnl ? (br ? 1 : 4) : 3,
+                      length, ops, nops);
+}
+
+int enqueue_theta(Session *s, const gems_branch *br) {
+  return launch_terms(s, br, kStore, 2, br->length, nullptr, 0);
 }
 
 // a non-finite total: the sum with non-finite pattern values clamped to 4 log(2^-256)

@@ -347,16 +347,20 @@ static int run_ops(Session *s, const gems_op *ops, int nops) {
 }
 
 // The node updates of a branch call: run here, or (short lists, small_ops) left to the launch
-// that follows, which is then given the first `*left` of them.
+// that follows, which is then given the first `*left` of them.  Kernel timing has an id for
+// traversals and one for theta: a session that is timed runs both in launches of their own.
 static int run_branch_ops(Session *s, const gems_op *ops, int nops, int *left) {
   *left = 0;
-  if (!small_ops(s, nops)) return run_ops(s, ops, nops);
+  if (!small_ops(s, nops) || s->prof_on) return run_ops(s, ops, nops);
   if (int st = check_ready(s)) return st;
   if (int st = check_ops(s, ops, nops)) return st;
   invalidate_theta(s, ops, nops);
   *left = nops;
   return GEMS_OK;
 }
+
+// whether the launch that uses a branch's theta forms it
+static bool forms_theta(const Session *s) { return theta_in_kernel(s) && !s->prof_on; }
 
 static void theta_of(Session *s, const gems_branch *br) {
   s->theta_valid = true;
@@ -370,8 +374,9 @@ static int start_theta(Session *s, const gems_op *ops, int nops, const gems_bran
                        int *left) {
   if (int st = run_branch_ops(s, ops, nops, left)) return st;
   s->theta_valid = false;
-  if (theta_in_kernel(s)) return GEMS_OK;
-  if (int st = enqueue_theta_mixed(s, br, false, true)) return st;
+  if (forms_theta(s)) return GEMS_OK;
+  if (int st = theta_in_kernel(s) ? enqueue_theta(s, br) : enqueue_theta_mixed(s, br, false, true))
+    return st;
   theta_of(s, br);
   return GEMS_OK;
 }
@@ -1068,7 +1073,7 @@ int gems_branch_derv(gems_session *s, const gems_op *ops, int nops, const gems_b
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
-  const bool form = compute_theta && theta_in_kernel(s);
+  const bool form = compute_theta && forms_theta(s);
   if ((st = launch_derv(s, form ? br : nullptr, br->length, df, ddf, ops, left))) return st;
   if (compute_theta) theta_of(s, br);
   if (df_frac) {
@@ -1107,7 +1112,7 @@ int gems_newton_branch_async(gems_session *s, const gems_op *ops, int nops,
     set_error("theta not computed");
     return GEMS_ERR_STATE;
   }
-  const bool form = compute_theta && theta_in_kernel(s);
+  const bool form = compute_theta && forms_theta(s);
   if ((st = launch_newton_async(s, form ? br : nullptr, br->length, min_len, max_len, xacc,
                                 max_steps, ops, left)))
     return st;

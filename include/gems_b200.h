@@ -287,7 +287,9 @@ int gems_launch_count(gems_session *s, long long *count);
 /* Kernel timing with CUDA events on the session stream: when enabled, every launch of the
  * traversal kernel (kernel id 0), branch kernel (1), theta (2), derivative (3),
  * from-buffer (4) and Newton (5) kernels is bracketed by events; gems_profile_read returns the
- * summed device time in ms and the number of timed launches, then resets the counters. */
+ * summed device time in ms and the number of timed launches, then resets the counters.  While
+ * enabled, the node updates and theta that a branch call otherwise has its own kernel do run in
+ * launches of their own, so that each id has its time; results are the same bits. */
 int gems_profile_enable(gems_session *s, int on);
 int gems_profile_read(gems_session *s, int kernel_id, double *total_ms, long long *launches);
 /* Alignment ingest on the device: state encoding and pattern compression in the reference's

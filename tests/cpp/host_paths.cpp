@@ -139,6 +139,38 @@ CASE(ingest_device_address) {
   gems_ingest_destroy(g);
 }
 
+// ---- kernel timing: every traversal counts under id 0, every theta under id 2 ------------------
+void profile_counts(int nstates, int ncat, int precision) {
+  gems_session *s = session(nstates, ncat, 300, precision, GEMS_SCALE_SAFE);
+  const std::vector<gems_op> ops = updates(3);
+  double a, b;
+  int n;
+  auto launches = [&](int id) {
+    double ms = 0.0;
+    long long k = 0;
+    EXPECT(gems_profile_read(s, id, &ms, &k) == GEMS_OK);
+    return (int)k;
+  };
+  EXPECT(gems_profile_enable(s, 1) == GEMS_OK);
+  EXPECT(gems_branch_derv(s, ops.data(), 3, &kBranch, 1, &a, &b, nullptr) == GEMS_OK);
+  EXPECT(launches(0) == 1 && launches(1) == 0 && launches(2) == 1 && launches(3) == 1);
+  EXPECT(gems_newton_branch(s, ops.data(), 3, &kBranch, 1, 1e-6, 10.0, 1e-6, 5, &a, &n) ==
+         GEMS_OK);
+  EXPECT(launches(0) == 1 && launches(2) == 1 && launches(5) == 1);
+  EXPECT(gems_lnl_from_buffer(s, 0.1, &a, nullptr) == GEMS_OK && launches(4) == 1);
+  EXPECT(gems_branch_lnl(s, ops.data(), 3, &kBranch, &a, nullptr) == GEMS_OK);
+  EXPECT(launches(0) == 1 && launches(1) == 1 && launches(2) == 0);
+  EXPECT(gems_profile_enable(s, 0) == GEMS_OK);
+  EXPECT(gems_branch_derv(s, ops.data(), 3, &kBranch, 1, &a, &b, nullptr) == GEMS_OK);
+  for (int id = 0; id < 6; id++) EXPECT(launches(id) == 0);
+  EXPECT(gems_session_destroy(s) == GEMS_OK);
+}
+CASE(profile_4_fp64) { profile_counts(4, 4, GEMS_PREC_FP64); }
+CASE(profile_4_mixed) { profile_counts(4, 4, GEMS_PREC_MIXED); }
+CASE(profile_20_fp64) { profile_counts(20, 4, GEMS_PREC_FP64); }
+CASE(profile_20_mixed) { profile_counts(20, 4, GEMS_PREC_MIXED); }
+CASE(profile_61_fp64) { profile_counts(61, 4, GEMS_PREC_FP64); }
+
 }  // namespace
 
 int main(int argc, char **argv) {
