@@ -183,7 +183,8 @@ struct Session {
   unsigned int *d_bar = nullptr;  // count of finished blocks of a branch-term launch (zero between)
   void *d_slots = nullptr;        // the Newton kernel's exchange slots
   unsigned int newton_launches = 0;
-  int newton_fit[2][2] = {{-1, -1}, {-1, -1}};  // clusters of 8, 16 the GPU holds, per kernel form
+  // clusters of 8 and of 16 that the GPU holds, per kernel form; the same of 8 streaming blocks
+  int newton_fit[2][2] = {{-1, -1}, {-1, -1}}, stream_fit = -1;
   // batched launches led by this session: job table (device and pinned host copies)
   static constexpr int kMaxBatch = 128;
   TcJob *d_jobs = nullptr;

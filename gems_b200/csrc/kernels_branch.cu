@@ -59,7 +59,7 @@ inline Split split_of(int B, int C) {
   while (L < C) L *= 2;
   while (L < 32 && (u + L - 1) / L > 5) L *= 2;
   const int need = (u + L - 1) / L;
-  for (int e : {1, 2, 3, 4, 5, 8})
+  for (int e : {1, 2, 3, 4, 5, 8, 12})
     if (need <= e) return {L, e};
   return {L, 16};  // 61 states, 16 categories: 488 pairs on 32 lanes
 }
@@ -272,6 +272,20 @@ __device__ __forceinline__ double dot(const double (&th)[2 * E2], const double *
     s = fma(w.y, th[2 * q + 1], s);
   }
   return s;
+}
+// the same of two patterns' elements, with one read of the table
+template <int E2>
+__device__ __forceinline__ void dot2(const double (&a)[2 * E2], const double (&b)[2 * E2],
+                                     const double *v, int L, int l, double &x, double &y) {
+  x = y = 0.0;
+#pragma unroll
+  for (int q = 0; q < E2; q++) {
+    const double2 w = *reinterpret_cast<const double2 *>(v + 2 * pair_of<E2>(q, l, L));
+    x = fma(w.x, a[2 * q], x);
+    y = fma(w.x, b[2 * q], y);
+    x = fma(w.y, a[2 * q + 1], x);
+    y = fma(w.y, b[2 * q + 1], y);
+  }
 }
 // x of the first pattern, y of the second: even lanes end with x's sum over the pattern's lanes,
 // odd lanes with y's (one exchange fewer than two sums)
@@ -729,32 +743,41 @@ struct NewtonArgs {
   double *result;            // pinned host memory: length, evaluations, status
 };
 
-// threads per block: more than five pairs per lane need more than 128 registers
+// threads of a block that takes an SM's registers: more than five pairs per lane need more than
+// 128 each
 __host__ __device__ constexpr int newton_threads(int e2) { return e2 <= 5 ? 512 : 256; }
 template <int E2>
 __host__ __device__ constexpr int held_rows() {
   return E2 <= 2 ? 4 : 2;  // an even number
 }
+// the same of blocks that hold no rows, and how many of them an SM takes
+__host__ __device__ constexpr int stream_threads(int e2) { return e2 <= 5 ? 256 : 128; }
+__host__ __device__ constexpr int stream_ctas(int e2) {
+  return e2 <= 2 || e2 == 8 || e2 == 12 ? 4 : 3;
+}
 
-template <int SRC, bool SAFE, int E2>
-__global__ void __launch_bounds__(newton_threads(E2), 1)
+// HELD: the first rows of each thread in registers, one block to an SM; else none (launched for
+// small shares of the GPU)
+template <int SRC, bool SAFE, int E2, bool HELD>
+__global__ void __launch_bounds__(HELD ? newton_threads(E2) : stream_threads(E2),
+                                  HELD ? 1 : stream_ctas(E2))
     k_newton(DevCtx c, const NewtonArgs a, const __grid_constant__ SmallOps ops) {
-  constexpr int kThreadsN = newton_threads(E2), kWarps = kThreadsN / 32;
   extern __shared__ __align__(16) double tab[];
-  __shared__ __align__(16) double2 recv[2][kMaxCluster * kWarps];
+  constexpr int nt = HELD ? newton_threads(E2) : stream_threads(E2), nw = nt / 32;
+  __shared__ __align__(16) double2 recv[2][kMaxCluster * nw];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ double tot[2];
   __shared__ bool tot_ok;
-  constexpr int RH = held_rows<E2>();
+  constexpr int RH = HELD ? held_rows<E2>() : 0, RA = RH ? RH : 2;
   constexpr double thr = SRC == kM4 ? kLogScaleThrF : kLogScaleThr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int CS = a.cluster, nclusters = gridDim.x / CS, rank = blockIdx.x % CS;
   const int L = a.L, len = 2 * L * E2, l = threadIdx.x & (L - 1);
-  const long per = kThreadsN / L, step = per * gridDim.x;
+  const long per = nt / L, step = per * gridDim.x;
   const long b0 = (long)blockIdx.x * per;
   const int sub = threadIdx.x / L;
-  const uint32_t s_recv = tc::sptr(&recv[0][0]), s_bars = tc::sptr(&bars[0]);
-  const uint32_t expect = CS * kWarps * sizeof(double2);
+  const uint32_t s_bars = tc::sptr(&bars[0]);
+  const uint32_t expect = CS * nw * sizeof(double2);
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; i++) {
       tc::mbar_init(s_bars + 8 * i, 1);
@@ -765,10 +788,10 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
   // the others' barriers are ready once all blocks have been here (waited for below)
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
-  const double *small = tab + 3 * len;
+  double *small = tab + 3 * len;
   if constexpr (small_form<SRC, E2>())
     if (ops.n) {
-      small_tables<SRC>(c, ops, tab + 3 * len);
+      small_tables<SRC>(c, ops, small);
       __syncthreads();
     }
   auto updates = [&](const long (&p)[2]) {
@@ -778,7 +801,7 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
 
   // theta of this thread's rows: formed and stored (or read), the first ones kept; of each two
   // patterns, even lanes hold the first's +I term and weight and odd lanes the second's
-  double th[RH][2 * E2], inva[RH / 2], fr[RH / 2];
+  double th[RA][2 * E2], inva[RA / 2], fr[RA / 2];
   auto weights = [&](long p, double &iv, double &f) {
     iv = f = 0.0;
     if (l < 2 && p < c.nptn) iv = c.invar[p], f = c.freq[p];
@@ -818,30 +841,48 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
       keep(p, v, m);
     }
 
-  // this thread's table elements (at most 2 x 32 x E2 of them)
-  constexpr int kTab = (64 * E2 + kThreadsN - 1) / kThreadsN;
+  // this thread's table elements: eval_i r_c and prop_c (HELD: at most 2 x 32 x E2 of them, else
+  // behind the tables)
+  constexpr int kTab = HELD ? (64 * E2 + nt - 1) / nt : 1;
   double cof[kTab], prop[kTab];
+  double2 *fac = reinterpret_cast<double2 *>(tab + 3 * len);
+  if constexpr (HELD) {
 #pragma unroll
-  for (int i = 0; i < kTab; i++) table_factors(c, threadIdx.x + i * kThreadsN, cof[i], prop[i]);
+    for (int i = 0; i < kTab; i++) table_factors(c, threadIdx.x + i * nt, cof[i], prop[i]);
+  } else {
+    for (int j = threadIdx.x; j < len; j += nt) table_factors(c, j, fac[j].x, fac[j].y);
+  }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   int nevals = 0;
   // f = -dlnL/dt and df = -d2lnL/dt2 at t (computeFuncDerv, phylotree.cpp:2555).  Tables of the
   // last evaluation may be overwritten: its sums have come, so every warp had read them.
   auto eval = [&](double t, double &f, double &df) -> bool {
+    if constexpr (HELD) {
 #pragma unroll
-    for (int i = 0; i < kTab; i++)
-      if (threadIdx.x + i * kThreadsN < len)
-        put_tables(t, threadIdx.x + i * kThreadsN, cof[i], prop[i], len, 3, tab);
+      for (int i = 0; i < kTab; i++)
+        if (threadIdx.x + i * nt < len)
+          put_tables(t, threadIdx.x + i * nt, cof[i], prop[i], len, 3, tab);
+    } else {
+      for (int j = threadIdx.x; j < len; j += nt) put_tables(t, j, fac[j].x, fac[j].y, len, 3, tab);
+    }
     __syncthreads();
     double v0 = 0.0, v1 = 0.0;
     // two patterns' terms, b and b + step from this block's start
     auto add = [&](const double (&x)[2 * E2], const double (&y)[2 * E2], long b, double iv,
                    double w) {
       const double *t1 = tab + len, *t2 = t1 + len;
-      const double h = lanes_sum2(dot<E2>(x, tab, L, l), dot<E2>(y, tab, L, l), L, l);
-      const double d = lanes_sum2(dot<E2>(x, t1, L, l), dot<E2>(y, t1, L, l), L, l);
-      const double g = lanes_sum2(dot<E2>(x, t2, L, l), dot<E2>(y, t2, L, l), L, l);
+      double h, d, g;
+      if constexpr (HELD) {
+        h = lanes_sum2(dot<E2>(x, tab, L, l), dot<E2>(y, tab, L, l), L, l);
+        d = lanes_sum2(dot<E2>(x, t1, L, l), dot<E2>(y, t1, L, l), L, l);
+        g = lanes_sum2(dot<E2>(x, t2, L, l), dot<E2>(y, t2, L, l), L, l);
+      } else {
+        double p, q;
+        dot2<E2>(x, y, tab, L, l, p, q), h = lanes_sum2(p, q, L, l);
+        dot2<E2>(x, y, t1, L, l, p, q), d = lanes_sum2(p, q, L, l);
+        dot2<E2>(x, y, t2, L, l, p, q), g = lanes_sum2(p, q, L, l);
+      }
       if (l < 2 && b + l * step + sub < c.nptn) {
         const double inv = 1.0 / (fabs(h) + iv);
         const double dff = d * inv, q = dff * w;
@@ -868,12 +909,12 @@ __global__ void __launch_bounds__(newton_threads(E2), 1)
     nevals++;
     const uint32_t bar = s_bars + 8 * set;
     if (lane < CS)
-      send_pair(cluster_addr(s_recv + (set * kMaxCluster * kWarps + rank * kWarps + warp) * 16, lane),
-                cluster_addr(bar, lane), v0, v1);
+      send_pair(cluster_addr(tc::sptr(&recv[set][rank * nw + warp]), lane), cluster_addr(bar, lane),
+                v0, v1);
     bool ok = cluster_wait(bar, use);
     v0 = v1 = 0.0;
     if (ok)
-      for (int i = lane; i < CS * kWarps; i += 32) {
+      for (int i = lane; i < CS * nw; i += 32) {
         const double2 v = recv[set][i];
         v0 += v.x;
         v1 += v.y;
@@ -962,7 +1003,7 @@ struct Fns {
 };
 template <int SRC, bool SAFE, int E2>
 Fns fns() {
-  return {(const void *)k_terms<SRC, SAFE, E2>, (const void *)k_newton<SRC, SAFE, E2>};
+  return {(const void *)k_terms<SRC, SAFE, E2>, (const void *)k_newton<SRC, SAFE, E2, true>};
 }
 template <int SRC, bool SAFE>
 Fns pick4(int e2) {  // 4 states: one or two pairs per lane
@@ -974,6 +1015,7 @@ Fns pick(int e2) {  // the pairs per lane that split_of gives for 20 and 61 stat
   if (e2 == 4) return fns<SRC, SAFE, 4>();
   if constexpr (SRC == kR61) {
     if (e2 == 8) return fns<SRC, SAFE, 8>();
+    if (e2 == 12) return fns<SRC, SAFE, 12>();
     if (e2 == 16) return fns<SRC, SAFE, 16>();
   }
   return fns<SRC, SAFE, 5>();
@@ -986,7 +1028,20 @@ Fns pick_mem(int e2) {
     case 4: return fns<kMem, false, 4>();
     case 5: return fns<kMem, false, 5>();
     case 8: return fns<kMem, false, 8>();
+    case 12: return fns<kMem, false, 12>();
     default: return fns<kMem, false, 16>();
+  }
+}
+const void *pick_stream(int e2) {
+  switch (e2) {
+    case 1: return (const void *)k_newton<kMem, false, 1, false>;
+    case 2: return (const void *)k_newton<kMem, false, 2, false>;
+    case 3: return (const void *)k_newton<kMem, false, 3, false>;
+    case 4: return (const void *)k_newton<kMem, false, 4, false>;
+    case 5: return (const void *)k_newton<kMem, false, 5, false>;
+    case 8: return (const void *)k_newton<kMem, false, 8, false>;
+    case 12: return (const void *)k_newton<kMem, false, 12, false>;
+    default: return (const void *)k_newton<kMem, false, 16, false>;
   }
 }
 Fns kernels_for(const Session *s, bool from_partials, int e2) {
@@ -1094,35 +1149,25 @@ int launch_newton_async(Session *s, const gems_branch *br, double guess, double 
                         double max_len, double xacc, int max_steps, const gems_op *ops,
                         int nops) {
   DevCtx c = s->ctx();
-  SmallOps o = small_list(ops, nops);
   const Split sp = split_of(s->block, s->desc.ncat);
-  const Fns f = kernels_for(s, br != nullptr, sp.E2);
+  const void *fn = kernels_for(s, br != nullptr, sp.E2).newton;
   int nsm = 0;
   GEMS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device));
-  const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * 3 +
-                                        small_doubles(nops, s->desc.ncat, mixed_of(s)));
-  const int threads = newton_threads(sp.E2);
+  const size_t table = sizeof(double) * 2 * sp.L * sp.E2;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeCooperative;  // all clusters of a launch resident together
   attr[1].val.cooperative = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3(newton_threads(sp.E2));
+  cfg.dynamicSmemBytes =
+      3 * table + sizeof(double) * small_doubles(nops, s->desc.ncat, mixed_of(s));
   cfg.stream = s->stream;
   cfg.attrs = attr;
-  // One block per SM at most, two patterns a thread where that fills them (a pair costs little
-  // more than one): one cluster of up to 16 blocks, which also holds up to the register rows of
-  // its threads, else clusters of 8, as many as the GPU takes at once.
-  const long per = threads / sp.L, held = sp.E2 <= 2 ? 4 : 2;
-  const int most = std::max(1, nsm / s->newton_share);
-  const long want = (s->P + 2 * per - 1) / (2 * per);
-  int *fits = s->newton_fit[br != nullptr];
-  auto fit = [&](int size) {  // clusters of 8 or 16 that the GPU holds at once
-    int &n = fits[size == 16];
+  auto fit = [&](int &n, int size) {  // clusters of this launch that the GPU holds at once
     if (n >= 0) return n;
-    if (size == 16 && cudaFuncSetAttribute(f.newton, cudaFuncAttributeNonPortableClusterSizeAllowed,
+    if (size == 16 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                            1) != cudaSuccess) {
       cudaGetLastError();
       return n = 0;
@@ -1131,23 +1176,56 @@ int launch_newton_async(Session *s, const gems_branch *br, double guess, double 
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(size);
     int m = 0;
-    if (cudaOccupancyMaxActiveClusters(&m, f.newton, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&m, fn, &cfg) != cudaSuccess) {
       cudaGetLastError();
       m = 0;
     }
     return n = m;
   };
-  const int one = most >= 16 && fit(16) > 0 ? 16 : 8;  // the largest single cluster
+  // One block per SM at most, two patterns a thread where that fills them (a pair costs little
+  // more than one): one cluster of up to 16 blocks, which also holds up to the register rows of
+  // its threads, else clusters of 8, as many as the GPU takes at once.
+  long per = cfg.blockDim.x / sp.L;
+  const long held = sp.E2 <= 2 ? 4 : 2;
+  int *fits = s->newton_fit[br != nullptr];
+  const int most = std::max(1, nsm / s->newton_share);
+  const long want = (s->P + 2 * per - 1) / (2 * per);
+  const int one = most >= 16 && fit(fits[1], 16) > 0 ? 16 : 8;  // the largest single cluster
   int cluster = 1, clusters = 1;
-  if (s->P <= one * per * held || most < 16 || fit(8) < 2) {
+  if (s->P <= one * per * held || most < 16 || fit(fits[0], 8) < 2) {
     while (cluster < want && 2 * cluster <= std::min(most, one)) cluster *= 2;
   } else {
     cluster = 8;
-    clusters = (int)std::min<long>({(want + 7) / 8, most / 8, fit(8), kMaxClusters});
+    clusters = (int)std::min<long>({(want + 7) / 8, most / 8, fits[0], kMaxClusters});
+  }
+  // A share of the GPU that does not hold all rows reads the others again in every evaluation.
+  // Blocks that hold none have more threads to an SM, and the same share of them is on more SMs;
+  // theta is formed before, by the whole GPU.  Clusters as small as the slots allow, so that few
+  // blocks of the share are lost to rounding.  A 16th of the GPU, blocks that hold rows / that
+  // hold none: 60,000 patterns of 4 states and 4 categories 221 / 102 us, 100,000 of 20 states
+  // 1,964 / 757, 8,000 of 61 states and 9 categories 5,232 / 1,396; a quarter 81 / 61, 520 / 253,
+  // 1,392 / 457.  Up to twice the rows that are held the extra launch outweighs it (18,501 patterns
+  // of 4 states on a quarter: 45.7 / 46.6).
+  if (s->newton_share > 1 && s->P > 2 * cluster * clusters * per * held) {
+    if (br)
+      if (int st = launch_terms(s, br, kStore, 2, br->length, ops, nops)) return st;
+    br = nullptr;
+    nops = 0;
+    fn = pick_stream(sp.E2);
+    cfg.blockDim = dim3(stream_threads(sp.E2));
+    cfg.dynamicSmemBytes = 5 * table;
+    per = cfg.blockDim.x / sp.L;
+    const int share = std::max(1, stream_ctas(sp.E2) * nsm / s->newton_share);
+    cluster = 1;
+    while (cluster < 8 && share > kMaxClusters * cluster) cluster *= 2;
+    clusters = (int)std::min<long>({(s->P + 2 * cluster * per - 1) / (2 * cluster * per),
+                                    share / cluster, kMaxClusters});
+    if (fit(s->stream_fit, 8) > 0) clusters = std::min(clusters, s->stream_fit * 8 / cluster);
   }
   attr[0].val.clusterDim.x = cluster;
   cfg.numAttrs = clusters > 1 ? 2 : 1;
   cfg.gridDim = dim3(cluster * clusters);
+  SmallOps o = small_list(ops, nops);
   NewtonArgs a{};
   if (br) a.br = *br;
   a.guess = guess;
@@ -1163,7 +1241,7 @@ int launch_newton_async(Session *s, const gems_branch *br, double guess, double 
   void *args[] = {&c, &a, &o};
   cudaEvent_t ev0;
   if (int st = prof_begin(s, 5, &ev0)) return st;
-  GEMS_CUDA(cudaLaunchKernelExC(&cfg, f.newton, args));
+  GEMS_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
   s->launches++;
   return prof_end(s, 5, ev0);
 }

@@ -113,10 +113,11 @@ enum { GEMS_OPT_TENSOR_CORES = 1, GEMS_OPT_TILED_FP64 = 2, GEMS_OPT_AUTOTUNE = 3
  * taking its tile two categories at a time with every internal child copied back from the
  * slot (no forwarding), instead of one CTA per SM with all categories at once; the values are
  * the same bits either way. */
-/* GEMS_OPT_NEWTON_SHARE (default 1): the device Newton loop (gems_newton_branch) is one
- * cooperative kernel whose blocks are all resident at once; with value k it takes at most 1/k
- * of the GPU's resident blocks, so that it runs beside other sessions' work instead of waiting
- * for the whole GPU (a server with many sessions sets k > 1).  Results do not change. */
+/* GEMS_OPT_NEWTON_SHARE (default 1): the device Newton loop (gems_newton_branch) is one kernel
+ * whose blocks (a cluster, or several in a cooperative launch) are all resident at once; with
+ * value k it takes at most 1/k of the GPU's resident blocks, so that it runs beside other sessions'
+ * work instead of waiting for the whole GPU (a server with many sessions sets k > 1).  Results do
+ * not change (but for the grouping of sums). */
 /* GEMS_OPT_AUTOTUNE (default 1): the first traversal of a 4-state session class (precision,
  * scaling, categories, pattern count to the power of two) with at least 2^22 pattern-updates
  * times every launch shape of the traversal kernel (patterns per lane group x blocks per SM; all

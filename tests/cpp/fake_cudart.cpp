@@ -185,15 +185,14 @@ cudaError_t cudaFuncSetAttribute(const void *fn, cudaFuncAttribute, int) {
   use(fn);
   return cudaSuccess;
 }
-// a block of 512 threads takes an SM's registers
+// 1,024 threads to an SM, of any kernel
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *, int threads,
                                                           size_t) {
-  *n = threads < 512 ? 512 / threads : 1;
+  *n = 1024 / threads;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunchConfig_t *c) {
-  const int per = c->blockDim.x < 512 ? 512 / c->blockDim.x : 1;
-  *n = 148 * per / (int)c->gridDim.x;
+  *n = 148 * (1024 / (int)c->blockDim.x) / (int)c->gridDim.x;
   return cudaSuccess;
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {

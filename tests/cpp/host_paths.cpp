@@ -3,6 +3,7 @@
 // usage: host_paths CASE (none: lists them); prints OK or the expectation that failed.
 #include <sys/mman.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -170,6 +171,27 @@ CASE(profile_4_mixed) { profile_counts(4, 4, GEMS_PREC_MIXED); }
 CASE(profile_20_fp64) { profile_counts(20, 4, GEMS_PREC_FP64); }
 CASE(profile_20_mixed) { profile_counts(20, 4, GEMS_PREC_MIXED); }
 CASE(profile_61_fp64) { profile_counts(61, 4, GEMS_PREC_FP64); }
+
+// ---- Newton loops under a share of the GPU: within it, on as many SMs as its blocks can take ---
+CASE(newton_share) {
+  const std::vector<gems_op> ops = updates(3);
+  double a;
+  int n;
+  for (int share : {2, 4, 16, 64})
+    for (int form = 0; form < 3; form++) {
+      const int states[] = {4, 20, 61}, cats[] = {8, 4, 16}, ptn[] = {400000, 100000, 20000};
+      gems_session *s = session(states[form], cats[form], ptn[form], GEMS_PREC_FP64, GEMS_SCALE_SAFE);
+      EXPECT(gems_session_set_option(s, GEMS_OPT_NEWTON_SHARE, share) == GEMS_OK);
+      fake::launches.clear();
+      EXPECT(gems_newton_branch(s, ops.data(), 3, &kBranch, 1, 1e-6, 10.0, 1e-6, 5, &a, &n) ==
+             GEMS_OK);
+      const fake::Launch &l = fake::launches.back();
+      EXPECT(l.kernel.find("k_newton") != std::string::npos);
+      const int blocks = (form == 0 ? 4 : 3) * 148 / share;  // of the blocks that fit the GPU
+      EXPECT(l.grid <= blocks && l.grid >= std::min(256, blocks) / 8 * 8);
+      EXPECT(gems_session_destroy(s) == GEMS_OK);
+    }
+}
 
 }  // namespace
 
