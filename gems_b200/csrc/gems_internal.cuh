@@ -295,11 +295,11 @@ int traverse_v2_wave_patterns(const Session *s);
 // launch shape of the 4-state traversal in use for this session's class (patterns per lane
 // group, blocks per SM); returns 1 while the tuner has not chosen yet, else 0
 int traverse_v2_shape(const Session *s, int *patterns_per_group, int *blocks_per_sm);
-// FP64 20-state traversal (kernels_f20.cu): op tables, traversal, and the kernel with its threads
-// and patterns per CTA
+// FP64 20-state traversal (kernels_f20.cu): op tables, traversal, and the kernel for n patterns
+// with its threads and patterns per CTA
 int launch_prep_ops_f20(Session *s, int nops);
 int launch_traverse_f20(Session *s, int nops, int p0, int p1);
-const void *traverse_f20_kernel(const Session *s, int *threads, int *patterns);
+const void *traverse_f20_kernel(const Session *s, int n, int *threads, int *patterns);
 // tcgen05 split-TF32 traversal for 20 states (kernels_tc.cu)
 size_t tc20_op_floats(int ncat, int unknown);
 bool tc20_supported(const Session *s);

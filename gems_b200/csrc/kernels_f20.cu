@@ -140,19 +140,31 @@ __device__ __forceinline__ int abs_hi(double x) {
   return h > 0x7ff00000 ? 0 : h;
 }
 
-// KC categories held in registers, CB of them per pass; MULTI: C > KC categories, KC at a time
-// (nothing forwarded: they share the registers), else C == KC
-template <bool SAFE, int KC, bool MULTI>
-__global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
+// Warps of a CTA, and CTAs on an SM, when W warps share a group of patterns
+__host__ __device__ constexpr int warps_f(int w) { return w == 3 ? 3 : kWarpsF; }
+__host__ __device__ constexpr int ctas_f(int w) { return w == 3 ? 5 : kCtasF; }
+
+// KC categories held in registers, CB of them per pass.  W warps share 8 patterns: 1: C == KC;
+// more: C > KC, `share` categories to each (the pattern's maximum, NORM, is exchanged in shared
+// memory); 0: C > KC and one warp for all, KC at a time (nothing forwarded: they share the
+// registers).
+template <bool SAFE, int KC, int W>
+__global__ void __launch_bounds__(32 * warps_f(W), ctas_f(W))
     k_traverse_f20(DevCtx c, const DevOp *__restrict__ ops, int nops,
-                   const double *__restrict__ tab, size_t stride, int p0, int p1) {
+                   const double *__restrict__ tab, size_t stride, int p0, int p1, int share) {
+  constexpr bool MULTI = W == 0;
+  constexpr int kGroups = W > 1 ? warps_f(W) / W : kWarpsF;
   constexpr int CB = KC < kPassF ? KC : kPassF;
   __shared__ double frag[2][15][32];  // evec, inv_evec as B fragments
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const long p = p0 + ((long)blockIdx.x * kWarpsF + (threadIdx.x >> 5)) * kPatF + g;
+  __shared__ int group_max[W > 1 ? kGroups : 1][W > 1 ? W : 1][kPatF];
+  const int warp = threadIdx.x >> 5, group = W > 1 ? warp / W : warp;
+  const long p = p0 + ((long)blockIdx.x * kGroups + group) * kPatF + g;
   const bool act = p < p1;
-  const int C = MULTI ? c.C : KC, blk = C * kN;
-  for (int i = threadIdx.x; i < 2 * 15 * 32; i += 32 * kWarpsF) {
+  const int C = W == 1 ? KC : c.C, blk = C * kN;
+  const int first_c = W > 1 ? warp % W * share : 0;             // this warp's categories
+  const int mine = W > 1 ? min(share, C - first_c) : KC;
+  for (int i = threadIdx.x; i < 2 * 15 * 32; i += 32 * warps_f(W)) {
     const int l = i & 31, sm = (i >> 5) % 15, s = sm / 3, m = sm % 3, n = l >> 2;
     // column n of tile m
     const int x = m < 2 ? 8 * m + n : 16 + (n >> 1);
@@ -200,13 +212,15 @@ __global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
           s_norm += c.scale[(size_t)id[i] * c.slot_scale + p];
     }
     double *dst = part + (size_t)op.dst_slot * c.slot_elems + (size_t)p * blk;
-    for (int c0 = 0; c0 < C; c0 += KC) {
+    for (int c0 = first_c; c0 < (MULTI ? C : first_c + 1); c0 += KC) {
 #pragma unroll
       for (int cb = 0; cb < KC; cb += CB) {
         // categories c0 + cb .. + nc of this pass (CB of them unless the last of an odd KC or C)
         const int cc = c0 + cb;
-        const int nc = MULTI ? min(CB, C - cc) : (KC - cb < CB ? KC - cb : CB);
-        if (MULTI && nc <= 0) break;
+        const int nc = MULTI   ? min(CB, C - cc)
+                       : W > 1 ? min(CB, mine - cb)
+                               : (KC - cb < CB ? KC - cb : CB);
+        if (W != 1 && nc <= 0) break;
         double v[2][CB][5];
         int sc[CB];
 #pragma unroll
@@ -291,6 +305,12 @@ __global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
       if (!SAFE && !MULTI) {
         hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, 1));
         hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, 2));
+        if constexpr (W > 1) {
+          if (t == 0) group_max[group][warp % W][g] = hmax;
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < W; i++) hmax = max(hmax, group_max[group][i][g]);
+        }
         sx[0] = s_norm;
         if (!tiptip && hmax < kThrHi && inv0) {
 #pragma unroll
@@ -302,7 +322,7 @@ __global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
         s_norm = sx[0];
       }
       if (act) {
-        const int nc = MULTI ? min(KC, C - c0) : KC;
+        const int nc = MULTI ? min(KC, C - c0) : mine;
         store_rows<KC>(dst + c0 * kN, t, nc, x);
         if (SAFE && t == 0) {
           uint16_t *q = c.scale + (size_t)op.dst_slot * c.slot_scale + (size_t)p * C + c0;
@@ -324,9 +344,14 @@ __global__ void __launch_bounds__(32 * kWarpsF, kCtasF)
         s_norm += 1;
       }
     }
-    if (!SAFE && act && t == 0)
+    if (!SAFE && act && t == 0 && first_c == 0)
       c.scale[(size_t)op.dst_slot * c.slot_scale + p] = (uint16_t)s_norm;
-    __syncwarp();  // the counters lane t = 0 wrote are read by its pattern's four lanes
+    // the counters that lane t = 0 wrote are read by its pattern's four lanes, with NORM by those
+    // of all the group's warps
+    if (!SAFE && W > 1)
+      __syncthreads();
+    else
+      __syncwarp();
     op = nxt;
     tl = tip_byte(op.l_kind, op.l_id);
     tr = tip_byte(op.r_kind, op.r_id);
@@ -383,23 +408,43 @@ __global__ void k_prep_ops_f20(DevCtx c, const DevOp *ops, double *tab, size_t s
 }
 
 template <bool SAFE>
-const void *kernel_f20(int C) {
-  switch (C) {
-    case 1: return (const void *)k_traverse_f20<SAFE, 1, false>;
-    case 2: return (const void *)k_traverse_f20<SAFE, 2, false>;
-    case 3: return (const void *)k_traverse_f20<SAFE, 3, false>;
-    case 4: return (const void *)k_traverse_f20<SAFE, 4, false>;
-    default: return (const void *)k_traverse_f20<SAFE, 4, true>;
+const void *kernel_f20(int C, int w) {
+  switch (w) {
+    case 0: return (const void *)k_traverse_f20<SAFE, 4, 0>;
+    case 2: return (const void *)k_traverse_f20<SAFE, 4, 2>;
+    case 3: return (const void *)k_traverse_f20<SAFE, 4, 3>;
+    case 4: return (const void *)k_traverse_f20<SAFE, 4, 4>;
   }
+  switch (C) {
+    case 1: return (const void *)k_traverse_f20<SAFE, 1, 1>;
+    case 2: return (const void *)k_traverse_f20<SAFE, 2, 1>;
+    case 3: return (const void *)k_traverse_f20<SAFE, 3, 1>;
+    default: return (const void *)k_traverse_f20<SAFE, 4, 1>;
+  }
+}
+
+// Warps that share a group of 8 patterns of n (W).  One warp for more than four categories is a
+// chain several times as long, with every child read back: 24 taxa, 16 categories, 100 patterns
+// 312 us (NORM; SAFE 345) against 121 (128) with four warps, 3,000 patterns 327 (362) against 168
+// (172); 5 categories, 100 patterns 134 (149) against 107.  Once the groups alone fill the GPU the
+// one warp, which reads each fragment of the matrices for more categories, is the faster: 100,000
+// patterns of 5 categories 1,012 us against 1,403, of 9 categories 1,674 against 2,042.  So the
+// warps share while all of them are resident at once.
+int warps_per_group(const Session *s, int n) {
+  const int C = s->desc.ncat, w = (C + 3) / 4;
+  if (w == 1) return 1;
+  const long groups = ((long)n + kPatF - 1) / kPatF;
+  return groups * w <= 148L * kCtasF * kWarpsF ? w : 0;
 }
 
 }  // namespace
 
-const void *traverse_f20_kernel(const Session *s, int *threads, int *patterns) {
-  *threads = 32 * kWarpsF;
-  *patterns = kPatF * kWarpsF;
-  return s->desc.scaling == GEMS_SCALE_SAFE ? kernel_f20<true>(s->desc.ncat)
-                                            : kernel_f20<false>(s->desc.ncat);
+const void *traverse_f20_kernel(const Session *s, int n, int *threads, int *patterns) {
+  const int w = warps_per_group(s, n);
+  *threads = 32 * warps_f(w);
+  *patterns = kPatF * (w > 1 ? warps_f(w) / w : kWarpsF);
+  return s->desc.scaling == GEMS_SCALE_SAFE ? kernel_f20<true>(s->desc.ncat, w)
+                                            : kernel_f20<false>(s->desc.ncat, w);
 }
 
 int launch_prep_ops_f20(Session *s, int nops) {
@@ -416,12 +461,15 @@ int launch_prep_ops_f20(Session *s, int nops) {
 int launch_traverse_f20(Session *s, int nops, int p0, int p1) {
   DevCtx c = s->ctx();
   int threads = 0, per = 0;
-  const void *fn = traverse_f20_kernel(s, &threads, &per);
+  const void *fn = traverse_f20_kernel(s, p1 - p0, &threads, &per);
   const int grid = (p1 - p0 + per - 1) / per;
   const DevOp *ops = s->d_ops;
   const double *tab = s->d_opmats;
   size_t stride = s->op_stride;
-  void *args[] = {&c, &ops, &nops, &tab, &stride, &p0, &p1};
+  // categories of a warp that shares its patterns: even counts of an even C (load_table)
+  const int C = s->desc.ncat, w = (C + 3) / 4;
+  int share = C % 2 ? (C + w - 1) / w : 4;
+  void *args[] = {&c, &ops, &nops, &tab, &stride, &p0, &p1, &share};
   GEMS_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, 0, s->stream));
   s->launches++;
   return GEMS_OK;

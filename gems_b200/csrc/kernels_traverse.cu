@@ -1629,7 +1629,7 @@ int traverse_v2_wave_patterns(const Session *s) {
   } else if (mixed) {
     fn = safe ? (const void *)k_traverse_mix<20, true> : (const void *)k_traverse_mix<20, false>;
   } else {
-    fn = traverse_f20_kernel(s, &threads, &per_block);
+    fn = traverse_f20_kernel(s, s->P, &threads, &per_block);
   }
   int nsm = 0, per_sm = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device) != cudaSuccess ||

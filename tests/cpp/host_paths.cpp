@@ -193,6 +193,21 @@ CASE(newton_share) {
     }
 }
 
+// ---- FP64 20-state traversals of few patterns: four categories to a warp, not all of them -------
+CASE(protein_few_patterns) {
+  const std::vector<gems_op> ops = updates(3);
+  for (int ncat = 1; ncat <= 16; ncat++)
+    for (int ptn : {1, 100, 3000}) {
+      gems_session *s = session(20, ncat, ptn, GEMS_PREC_FP64, GEMS_SCALE_NORM);
+      fake::launches.clear();
+      EXPECT(gems_traverse(s, ops.data(), 3) == GEMS_OK);
+      const fake::Launch &l = fake::launches.back();
+      EXPECT(l.kernel.find("k_traverse_f20") != std::string::npos);
+      EXPECT(l.grid * l.threads / 32 >= (ptn + 7) / 8 * ((ncat + 3) / 4));
+      EXPECT(gems_session_destroy(s) == GEMS_OK);
+    }
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
