@@ -75,7 +75,8 @@ def measure_peaks(device=0):
 
 
 def check_barrier_timeout(device=0):
-    """Status the grid barrier reports when a wait cannot complete (GEMS_ERR_TIMEOUT = 4)."""
+    """Status that the Newton loop's waits report when they cannot complete (GEMS_ERR_TIMEOUT
+    = 4: both ran out)."""
     st = c_int()
     _check(_lib.gems().gems_check_barrier_timeout(device, byref(st)), "check_barrier_timeout")
     return st.value

@@ -734,6 +734,34 @@ __device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
+// The cluster wait's time-out path on purpose: two blocks send each other a pair and wait for one
+// more, so each gives up after the clock budget.  The flag reads GEMS_ERR_TIMEOUT when they did
+// and the pairs that were sent have come.
+__global__ void k_cluster_probe(int *flag) {
+  __shared__ __align__(16) double2 recv[2];
+  __shared__ __align__(8) uint64_t bar;
+  const uint32_t s_bar = tc::sptr(&bar);
+  const int rank = blockIdx.x & 1;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(s_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect_tx(s_bar, 3 * sizeof(double2));
+    recv[0] = recv[1] = make_double2(0.0, 0.0);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x < 2)
+    send_pair(cluster_addr(tc::sptr(&recv[rank]), threadIdx.x), cluster_addr(s_bar, threadIdx.x),
+              1.0, 2.0);
+  const bool ok = cluster_wait(s_bar, 0);
+  // the other block has given up too: nothing is on its way to this one
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const volatile double *v = &recv[0].x;
+  if (threadIdx.x == 0 && blockIdx.x == 0)
+    atomicExch(flag, !ok && v[0] + v[1] + v[2] + v[3] == 6.0 ? GEMS_ERR_TIMEOUT : GEMS_OK);
+}
+
 struct NewtonArgs {
   gems_branch br;
   double guess, x1, x2, xacc;
@@ -1251,20 +1279,34 @@ int check_barrier_timeout(int device, int *status) {
   ulonglong2 *slots = nullptr;
   int *flag = nullptr;
   GEMS_CUDA(cudaMalloc((void **)&slots, newton_slot_bytes()));
-  cudaError_t e = cudaMalloc((void **)&flag, sizeof(int));
+  cudaError_t e = cudaMalloc((void **)&flag, 2 * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(slots, 0, newton_slot_bytes());
-  if (e == cudaSuccess) e = cudaMemset(flag, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(flag, 0, 2 * sizeof(int));
   if (e == cudaSuccess) {
     void *args[] = {&slots, &flag};
     e = cudaLaunchCooperativeKernel((void *)k_exchange_probe, dim3(2), dim3(32), args, 0, nullptr);
   }
+  if (e == cudaSuccess) {
+    int *second = flag + 1;
+    void *args[] = {&second};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(32);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelExC(&cfg, (void *)k_cluster_probe, args);
+  }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  int h = -1;
-  if (e == cudaSuccess) e = cudaMemcpy(&h, flag, sizeof(int), cudaMemcpyDeviceToHost);
+  int h[2] = {-1, -1};
+  if (e == cudaSuccess) e = cudaMemcpy(h, flag, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(slots);
   cudaFree(flag);
   if (e != cudaSuccess) return cuda_status(e, "exchange probe");
-  *status = h;
+  *status = h[0] == GEMS_ERR_TIMEOUT ? h[1] : h[0];
   return GEMS_OK;
 }
 

@@ -208,6 +208,20 @@ CASE(protein_few_patterns) {
     }
 }
 
+// ---- the probe of the Newton loop's waits reports a time-out only when both ran out ------------
+CASE(wait_probe) {
+  for (int slots : {GEMS_OK, GEMS_ERR_TIMEOUT})
+    for (int cluster : {GEMS_OK, GEMS_ERR_TIMEOUT}) {
+      fake::on_launch = [=](const std::string &name, void **args) {
+        if (name.find("k_exchange_probe") != std::string::npos) **static_cast<int **>(args[1]) = slots;
+        if (name.find("k_cluster_probe") != std::string::npos) **static_cast<int **>(args[0]) = cluster;
+      };
+      int status = -1;
+      EXPECT(gems_check_barrier_timeout(0, &status) == GEMS_OK);
+      EXPECT((status == GEMS_ERR_TIMEOUT) == (slots && cluster));
+    }
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
