@@ -222,6 +222,43 @@ CASE(wait_probe) {
     }
 }
 
+// ---- the launch shape of large 4-state traversals is chosen by the kernels' time: neither what the
+// host does when a kernel is first used nor one launch that something else held up moves it ------
+const char *tuned_kernel(int precision, double pattern_ms, double staged_ms, double first_use,
+                         int held_up) {
+  gems_session *s = session(4, 4, 200000, precision, GEMS_SCALE_NORM, 32);
+  fake::first_use_ms = [=](const std::string &name) {  // the first of them loads the most
+    return name.find("k_traverse4p") != std::string::npos ? first_use : 0.5;
+  };
+  int full = 0;
+  fake::kernel_ms = [&](const std::string &name, const fake::Launch &l) {
+    const bool pattern = name.find("k_traverse4p") != std::string::npos;
+    if (!pattern && name.find("k_traverse4q") == std::string::npos) return 0.01;
+    if (l.grid < 100) return 0.5;  // a few patterns
+    if (pattern && full++ < held_up) return 30.0;
+    return pattern ? pattern_ms : staged_ms;
+  };
+  const std::vector<gems_op> ops = updates(31);
+  EXPECT(gems_traverse(s, ops.data(), 31) == GEMS_OK);
+  fake::launches.clear();
+  EXPECT(gems_traverse(s, ops.data(), 31) == GEMS_OK);
+  EXPECT(count("k_traverse4p") + count("k_traverse4q") == 1);  // tuned: one launch
+  const char *k = count("k_traverse4p") ? "pattern" : "staged";
+  EXPECT(gems_session_destroy(s) == GEMS_OK);
+  return k;
+}
+CASE(tuner_first_use) {
+  EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_MIXED, 6.0, 13.0, 25.0, 0), "pattern"));
+  EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_FP64, 6.0, 13.0, 25.0, 0), "pattern"));
+}
+CASE(tuner_held_up) {
+  EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_MIXED, 6.0, 13.0, 0.0, 1), "pattern"));
+}
+CASE(tuner_faster_shape) {
+  EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_MIXED, 13.0, 6.0, 25.0, 0), "staged"));
+  EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_FP64, 6.0, 5.95, 25.0, 0), "pattern"));  // within noise
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
