@@ -24,10 +24,12 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
                   "--expt-relaxed-constexpr", "-I" + INCLUDE, "-I" + CSRC]
 
-CUDA_SOURCES = ["session.cu", "kernels_fp64.cu", "kernels_branch.cu", "kernels_mixed.cu", "kernels_traverse.cu", "kernels_f20.cu",
+CUDA_SOURCES = ["session.cu", "kernels_fp64.cu", "kernels_branch.cu", "branch_f64_4.cu",
+                "branch_mixed_4.cu", "branch_f64_20.cu", "branch_f64_61.cu", "branch_f64_61_wide.cu",
+                "branch_memory_4.cu", "branch_memory_20.cu", "branch_memory_wide.cu", "kernels_mixed.cu", "kernels_traverse.cu", "kernels_f20.cu",
                 "kernels_tc20.cu", "kernels_tc61.cu", "kernels_g61.cu", "kernels_rell.cu", "eigen.cu", "noalloc.cu", "peaks.cu", "ingest.cu",
                 "phylotree.cpp"]
-HEADERS = ["gems_internal.cuh", "tc_common.cuh", "plan.h"]
+HEADERS = ["gems_internal.cuh", "tc_common.cuh", "branch_kernels.cuh", "plan.h"]
 
 LIB = os.path.join(HERE, "libgems_b200.so")
 SYNTH = os.path.join(HERE, "libgems_synth.so")

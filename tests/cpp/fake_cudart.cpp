@@ -19,10 +19,17 @@ std::set<const void *> device_only;
 std::function<void(const std::string &, void **)> on_launch;
 std::function<double(const std::string &, const Launch &)> kernel_ms;
 std::function<double(const std::string &)> first_use_ms;
+std::map<void **, std::vector<std::string>> &modules() {  // filled before main
+  static std::map<void **, std::vector<std::string>> m;
+  return m;
+}
 }  // namespace fake
 
 namespace {
-std::map<const void *, std::string> g_names;
+std::map<const void *, std::string> &names() {  // filled before main
+  static std::map<const void *, std::string> m;
+  return m;
+}
 std::set<const void *> g_used;
 std::map<void *, size_t> g_sizes;
 double g_host = 0.0, g_stream = 0.0;  // ms
@@ -37,10 +44,10 @@ cudaError_t check(const char *call) {
   return fake::fail_call == call ? cudaErrorUnknown : cudaSuccess;
 }
 void use(const void *fn) {
-  if (g_used.insert(fn).second && fake::first_use_ms) g_host += fake::first_use_ms(g_names[fn]);
+  if (g_used.insert(fn).second && fake::first_use_ms) g_host += fake::first_use_ms(names()[fn]);
 }
 cudaError_t launch(const void *fn, dim3 grid, dim3 block, void **args) {
-  const std::string &name = g_names[fn];
+  const std::string &name = names()[fn];
   if (!fake::fail_kernel.empty() && name.find(fake::fail_kernel) != std::string::npos)
     return g_last = cudaErrorCooperativeLaunchTooLarge;
   use(fn);
@@ -64,15 +71,13 @@ struct CUevent_st {
 };
 
 extern "C" {
-void **__cudaRegisterFatBinary(void *) {
-  static void *h;
-  return &h;
-}
+void **__cudaRegisterFatBinary(void *) { return new void *; }
 void __cudaRegisterFatBinaryEnd(void **) {}
 void __cudaUnregisterFatBinary(void **) {}
-void __cudaRegisterFunction(void **, const char *host, char *, const char *name, int, uint3 *,
+void __cudaRegisterFunction(void **module, const char *host, char *, const char *name, int, uint3 *,
                             uint3 *, dim3 *, dim3 *, int *) {
-  g_names[host] = name;
+  names()[host] = name;
+  fake::modules()[module].push_back(name);
 }
 void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {

@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <functional>
+#include <map>
 #include <set>
 #include <string>
 #include <vector>
@@ -15,6 +16,8 @@ struct Launch {
 extern std::vector<Launch> launches;
 // launches of kernels with this in their name fail; calls of this name fail ("" for none)
 extern std::string fail_kernel, fail_call;
+// kernels of each module (translation unit)
+std::map<void **, std::vector<std::string>> &modules();
 extern size_t allocated;                   // bytes of device memory held
 extern std::set<const void *> device_only;  // addresses the runtime takes for device memory
 // called for each launch with the kernel's arguments

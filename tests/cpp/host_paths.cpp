@@ -259,6 +259,20 @@ CASE(tuner_faster_shape) {
   EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_FP64, 6.0, 5.95, 25.0, 0), "pattern"));  // within noise
 }
 
+// ---- a module is loaded whole by the first launch of one of its kernels: the branch kernels, most
+// of the library's, come in modules of one kind of session each -----------------------------------
+CASE(branch_modules) {
+  int branch = 0;
+  for (const auto &m : fake::modules()) {
+    int here = 0;
+    for (const std::string &k : m.second)
+      here += k.find("k_terms") != std::string::npos || k.find("k_newton") != std::string::npos;
+    EXPECT(here <= 12);
+    branch += here;
+  }
+  EXPECT(branch >= 50);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {

@@ -26,7 +26,7 @@ def sources_that_send():
 
 
 def test_the_newton_exchange_is_covered():
-    assert [os.path.basename(p) for p in sources_that_send()] == ["kernels_branch.cu"]
+    assert [os.path.basename(p) for p in sources_that_send()] == ["branch_kernels.cuh"]
 
 
 @pytest.mark.parametrize("path", sources_that_send(), ids=os.path.basename)
