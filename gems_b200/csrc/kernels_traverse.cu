@@ -1531,12 +1531,26 @@ int shape4(const Session *s, bool mixed) {  // forced, tuned (-1: not yet), for 
   return s->force_shape >= 0 ? (s->force_shape < nv ? s->force_shape : nv - 1) : tuned4(s, mixed);
 }
 
+// whether the uploaded list gives the same partials when it is run again: no slot is written that
+// was read before (as the calls before this one left it)
+bool repeatable(const Session *s, int nops) {
+  std::vector<char> read(s->desc.nslots, 0), written(s->desc.nslots, 0);
+  for (int k = 0; k < nops; k++) {
+    const DevOp &o = s->h_ops[k];
+    if (o.l_kind == GEMS_CHILD_PARTIAL && !written[o.l_id]) read[o.l_id] = 1;
+    if (o.r_kind == GEMS_CHILD_PARTIAL && !written[o.r_id]) read[o.r_id] = 1;
+    if (read[o.dst_slot]) return false;
+    written[o.dst_slot] = 1;
+  }
+  return true;
+}
+
 int traverse4(Session *s, bool mixed, int nops, int p0, int p1, const EigPack<4> *E) {
   int nv = 0;
   variants4(mixed, &nv);
   const int v = shape4(s, mixed);
   const bool tune = v < 0 && s->autotune && p0 == 0 && p1 == s->P &&
-                    (long long)s->P * nops >= kTuneMinWork;
+                    (long long)s->P * nops >= kTuneMinWork && repeatable(s, nops);
   if (!tune) return launch4(s, mixed, v < 0 ? 0 : v, nops, p0, p1, E);
   // The shapes are timed on the stream, so nothing else may come between their events: a launch of
   // one op loads each kernel and looks up its limits first.  (That host work, tens of milliseconds

@@ -259,6 +259,23 @@ CASE(tuner_faster_shape) {
   EXPECT(!std::strcmp(tuned_kernel(GEMS_PREC_FP64, 6.0, 5.95, 25.0, 0), "pattern"));  // within noise
 }
 
+// a list that reads a slot and then writes it gives something else when it is run again: not tuned
+CASE(tuner_list_not_repeatable) {
+  gems_session *s = session(4, 4, 200000, GEMS_PREC_FP64, GEMS_SCALE_NORM, 32);
+  auto launches = [&](const std::vector<gems_op> &ops) {
+    fake::launches.clear();
+    EXPECT(gems_traverse(s, ops.data(), (int)ops.size()) == GEMS_OK);
+    return count("k_traverse4") + count("k_traverse_f64x");
+  };
+  std::vector<gems_op> ops = updates(31);
+  ops[0].left_kind = GEMS_CHILD_PARTIAL, ops[0].left_id = 30;  // as it was: written by the last op
+  EXPECT(launches(ops) == 1);
+  ops[0].left_id = 31;  // not written
+  EXPECT(launches(ops) > 1);
+  EXPECT(launches(ops) == 1);
+  EXPECT(gems_session_destroy(s) == GEMS_OK);
+}
+
 // ---- a module is loaded whole by the first launch of one of its kernels: the branch kernels, most
 // of the library's, come in modules of one kind of session each -----------------------------------
 CASE(branch_modules) {
