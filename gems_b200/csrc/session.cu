@@ -108,11 +108,14 @@ static int pow2_at_least(int x) {
   return g;
 }
 
+constexpr size_t kFlagBytes = 16 * sizeof(int);
+constexpr size_t kBarBytes = 128;  // the ticket of branch-term launches, then the Newton slots
+
 struct Sizes {
   bool tiled;
   size_t slot_elems;
-  size_t partial_bytes, scale_bytes, theta_bytes, opmats_bytes, branch_bytes, red_doubles,
-      model_doubles, total;
+  size_t partial_bytes, scale_bytes, theta_bytes, opmats_bytes, bar_bytes, red_doubles, model_doubles,
+      total;
   int nops_max;
   size_t op_stride;
 };
@@ -152,13 +155,13 @@ static Sizes compute_sizes(const gems_session_desc &d) {
   }
   z.op_stride = (z.op_stride + 7) & ~(size_t)7;  // 64-byte aligned op tables
   z.opmats_bytes = (size_t)z.nops_max * z.op_stride * sizeof(double);
-  z.branch_bytes = (3 * blk + (size_t)(unk + 1) * blk) * sizeof(double);
+  z.bar_bytes = kBarBytes + newton_slot_bytes();
   z.red_doubles = 4 * (P * 16 / 256 + 1024);
   z.model_doubles = d.nstates + 2 * (size_t)d.nstates * d.nstates + 2 * d.ncat +
                     2 * (size_t)(unk + 1) * d.nstates;
-  z.total = z.partial_bytes + z.scale_bytes + z.theta_bytes + z.opmats_bytes + z.branch_bytes +
+  z.total = z.partial_bytes + z.scale_bytes + z.theta_bytes + z.opmats_bytes + z.bar_bytes +
             z.red_doubles * 8 + z.model_doubles * 8 + (size_t)d.ntaxa * P + 2 * P * 8 +
-            (size_t)z.nops_max * sizeof(DevOp);
+            (size_t)z.nops_max * sizeof(DevOp) + sizeof(TcJob) * Session::kMaxBatch + kFlagBytes;
   return z;
 }
 
@@ -548,9 +551,9 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
   ALLOC(s->d_ops, (size_t)z.nops_max * sizeof(DevOp));
   ALLOC(s->d_opmats, z.opmats_bytes);
   ALLOC(s->d_red, z.red_doubles * sizeof(double));
-  ALLOC(s->d_flag, 16 * sizeof(int));
-  ALLOC(s->d_bar, 128 + newton_slot_bytes());  // then the Newton exchange's slots
-  s->d_slots = reinterpret_cast<char *>(s->d_bar) + 128;
+  ALLOC(s->d_flag, kFlagBytes);
+  ALLOC(s->d_bar, z.bar_bytes);
+  s->d_slots = reinterpret_cast<char *>(s->d_bar) + kBarBytes;
 #undef ALLOC
   if ((e = cudaHostAlloc((void **)&s->h_ops, (size_t)z.nops_max * sizeof(DevOp), 0)) !=
       cudaSuccess)
@@ -569,7 +572,7 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
       (e = cudaMemsetAsync(s->d_freq, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_invar, 0, P * sizeof(double), s->stream)) ||
       (e = cudaMemsetAsync(s->d_scale, 0, z.scale_bytes, s->stream)) ||
-      (e = cudaMemsetAsync(s->d_bar, 0, 128 + newton_slot_bytes(), s->stream)) ||
+      (e = cudaMemsetAsync(s->d_bar, 0, z.bar_bytes, s->stream)) ||
       (e = cudaStreamSynchronize(s->stream)))
     return fail(e, "initialise session");
   *out = s;

@@ -276,6 +276,22 @@ CASE(tuner_list_not_repeatable) {
   EXPECT(gems_session_destroy(s) == GEMS_OK);
 }
 
+// ---- a session's footprint is what it allocates --------------------------------------------------
+CASE(footprint) {
+  for (int nstates : {4, 20, 61})
+    for (int precision : {GEMS_PREC_FP64, GEMS_PREC_MIXED})
+      for (int ncat : {1, 4, 16}) {
+        gems_session_desc d{12, 777, nstates, ncat, 10, precision, GEMS_SCALE_SAFE, 0};
+        size_t bytes = 0;
+        EXPECT(gems_session_footprint(&d, &bytes) == GEMS_OK);
+        gems_session *s = nullptr;
+        EXPECT(gems_session_create(&d, &s) == GEMS_OK);
+        EXPECT(bytes == fake::allocated);
+        EXPECT(gems_session_destroy(s) == GEMS_OK);
+        EXPECT(fake::allocated == 0);
+      }
+}
+
 // ---- a module is loaded whole by the first launch of one of its kernels: the branch kernels, most
 // of the library's, come in modules of one kind of session each -----------------------------------
 CASE(branch_modules) {
