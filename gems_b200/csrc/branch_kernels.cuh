@@ -804,13 +804,14 @@ __global__ void __launch_bounds__(HELD ? newton_threads(E2) : stream_threads(E2)
     if (l < 2 && p < c.nptn) iv = c.invar[p], f = c.freq[p];
   };
   auto keep = [&](const long (&p)[2], const double (&v)[2][2 * E2], const int (&m)[2]) {
-    if (SRC == kMem) return;
+    if constexpr (SRC != kMem) {
 #pragma unroll
-    for (int u = 0; u < 2; u++)
-      if (p[u] < c.P) {
-        store_theta<E2>(c, L, l, p[u], v[u]);
-        if (l == 0) c.scale_all[p[u]] = (double)m[u] * thr;
-      }
+      for (int u = 0; u < 2; u++)
+        if (p[u] < c.P) {
+          store_theta<E2>(c, L, l, p[u], v[u]);
+          if (l == 0) c.scale_all[p[u]] = (double)m[u] * thr;
+        }
+    }
   };
 #pragma unroll
   for (int r = 0; r < RH; r += 2) {

@@ -138,6 +138,34 @@ __device__ __forceinline__ void store_row(double *__restrict__ slot, const DevCt
     for (int i = 0; i < N; i++) dst[i] = v[i];
   }
 }
+// d += a . b of one FP64 mma (m8n8k4): lane (g, t) = (lane / 4, lane % 4) holds A[g][k = t],
+// B[k = t][n = g] and D[g][2t], D[g][2t + 1]
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+// sums of K values over the block in a fixed tree, valid in thread 0
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[32]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    double x = v[k];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) sh[k][w] = x;
+  }
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double x = lane < nw ? sh[k][lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      v[k] = x;
+    }
+  }
+  __syncthreads();
+}
 #endif
 
 // one session of a batched tensor-core launch (sessions that share the op list: the same tree
@@ -155,6 +183,7 @@ struct Session {
   int block = 0;
   int G = 1;
   int nops_max = 0;
+  int nsm = 0;           // SMs of the device
   int plan_depth = 0;    // stack positions the uploaded op list's plan uses
   size_t op_stride = 0;  // doubles per op in opmats
   cudaStream_t stream = nullptr;

@@ -394,8 +394,9 @@ extern "C" int gems_ingest_create(int device, int ntaxa, long long nsites, int n
 
 // Makes the pages of a destination that a copy will fill.  A caller's fresh array has none yet,
 // and a device copy into it faults them in one by one (43 MB: 10 ms instead of 2.5); a few threads
-// take the faults side by side, by a write access that leaves every byte as it is.  Only pageable host memory: pinned memory has its pages, and an address
-// the host cannot write to is for the copy to refuse.
+// take the faults side by side, by a write access that leaves every byte as it is.  Only pageable
+// host memory: pinned memory has its pages, and an address the host cannot write to is for the
+// copy to refuse.
 static void touch_pages(uint8_t *p, size_t n) {
   constexpr size_t kPage = 4096, kLeast = 4u << 20;
   if (n < kLeast) return;

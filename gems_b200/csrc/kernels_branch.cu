@@ -97,7 +97,7 @@ static int launch_terms(Session *s, const gems_branch *br, int flags, int id, do
   Split sp = split_of(s->block, s->desc.ncat);
   const BranchFns f = kernels_for(s, br != nullptr, sp.E2);
   const long per = kThreadsT / sp.L;
-  const int grid = (int)std::min<long>(148 * ctas_t(sp.E2), (s->P + per - 1) / per);
+  const int grid = (int)std::min<long>(s->nsm * ctas_t(sp.E2), (s->P + per - 1) / per);
   gems_branch b{};
   if (br) b = *br;
   const size_t smem = sizeof(double) * (2 * sp.L * sp.E2 * (flags & kDerv ? 3 : 1) +
@@ -160,8 +160,7 @@ int launch_newton_async(Session *s, const gems_branch *br, double guess, double 
   DevCtx c = s->ctx();
   const Split sp = split_of(s->block, s->desc.ncat);
   const void *fn = kernels_for(s, br != nullptr, sp.E2).newton;
-  int nsm = 0;
-  GEMS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device));
+  const int nsm = s->nsm;
   const size_t table = sizeof(double) * 2 * sp.L * sp.E2;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -40,13 +40,6 @@ constexpr int kPassF = 2;            // categories per pass
 constexpr int kCtasF = 4;            // resident CTAs per SM (128 registers)
 constexpr int kThrHi = 0x2FF00000;   // high word of 2^-256
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile(
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
 // the state of K step s at lane position t
 __device__ __forceinline__ int state_of(int s, int t) {
   return s < 4 ? 8 * (s >> 1) + 2 * t + (s & 1) : 16 + t;
@@ -434,7 +427,7 @@ int warps_per_group(const Session *s, int n) {
   const int C = s->desc.ncat, w = (C + 3) / 4;
   if (w == 1) return 1;
   const long groups = ((long)n + kPatF - 1) / kPatF;
-  return groups * w <= 148L * kCtasF * kWarpsF ? w : 0;
+  return groups * w <= (long)s->nsm * kCtasF * kWarpsF ? w : 0;
 }
 
 }  // namespace

@@ -123,10 +123,8 @@ struct TileMap {
   __device__ size_t off(int r) const { return ((size_t)pattern(r) * C + cat(r)) * kN; }
 };
 
-// V of one child for the thread's rows and columns, and its scale counts (per row: SAFE; the
-// pattern's: NORM).  A partial child's GEMM leaves sA in use: the caller synchronises before
-// the next write of sA.
-template <bool SAFE>
+// V of one child for the thread's rows and columns, and their patterns' scale counts.  A partial
+// child's GEMM leaves sA in use: the caller synchronises before the next write of sA.
 __device__ __forceinline__ void child_v(const DevCtx &c, const TileMap &tm, int kind, int id,
                                         const double *et, const double *leaf, double *sA, int ty,
                                         int tx, double (&v)[8][4], int (&s)[8]) {
@@ -181,8 +179,7 @@ __device__ __forceinline__ void child_v(const DevCtx &c, const TileMap &tm, int 
 #pragma unroll
   for (int j = 0; j < 8; j++) {
     const int r = ty * 8 + j;
-    const long p = tm.pattern(r);
-    s[j] = tm.valid(r) ? (SAFE ? sc[(size_t)p * tm.C + tm.cat(r)] : sc[p]) : 0;
+    s[j] = tm.valid(r) ? sc[tm.pattern(r)] : 0;
   }
   __syncthreads();
   // rows past the tile's (64 % C) have no category: any table will do, their A rows are zero
@@ -190,14 +187,13 @@ __device__ __forceinline__ void child_v(const DevCtx &c, const TileMap &tm, int 
   gemm_tile<true>(sA, et + (size_t)cat * kK * kNC, ty, tx, v);
 }
 
-template <bool SAFE>
 __global__ void __launch_bounds__(kThreadsG, 2)
     k_traverse_g61(DevCtx c, const DevOp *__restrict__ ops, int nops,
                    const double *__restrict__ tab, size_t stride, int tile0) {
   extern __shared__ __align__(16) double smem[];
   double *sIv = smem;                  // [kK][kNC]: inv_evec[j][x] at [x][j]
   double *sA = sIv + kK * kNC;         // [kK][kSaLd]
-  double *sMax = sA + kK * kSaLd;      // [kRows] row maxima (NORM)
+  double *sMax = sA + kK * kSaLd;      // [kRows] row maxima
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   TileMap tm;
   tm.C = c.C;
@@ -222,9 +218,9 @@ __global__ void __launch_bounds__(kThreadsG, 2)
     double vl[8][4], o[8][4];
     int sl[8], sr[8];
     __syncthreads();  // sA free (previous op's last GEMM, or the set-up)
-    child_v<SAFE>(c, tm, op.l_kind, op.l_id, tk, leafL, sA, ty, tx, vl, sl);
+    child_v(c, tm, op.l_kind, op.l_id, tk, leafL, sA, ty, tx, vl, sl);
     __syncthreads();
-    child_v<SAFE>(c, tm, op.r_kind, op.r_id, tk + et_doubles(c.C), leafR, sA, ty, tx, o, sr);
+    child_v(c, tm, op.r_kind, op.r_id, tk + et_doubles(c.C), leafR, sA, ty, tx, o, sr);
     __syncthreads();
     // T = V_L (*) V_R into sA (k-major); columns >= 61 of V are zero, so row 61 of T is zero
 #pragma unroll
@@ -246,20 +242,18 @@ __global__ void __launch_bounds__(kThreadsG, 2)
       for (int off = 1; off < 16; off <<= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, off));
       m[j] = x;
     }
-    if (!SAFE) {
-      // the pattern's maximum over its C rows (rows c * tp + lp, in other threads)
-      if (tx == 0) {
+    // the pattern's maximum over its C rows (rows c * tp + lp, in other threads)
+    if (tx == 0) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) sMax[ty * 8 + j] = m[j];
-      }
-      __syncthreads();
+      for (int j = 0; j < 8; j++) sMax[ty * 8 + j] = m[j];
+    }
+    __syncthreads();
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int lp = (ty * 8 + j) % tm.tp;
-        double x = 0.0;
-        for (int u = 0; u < tm.C; u++) x = fmax(x, sMax[u * tm.tp + lp]);
-        m[j] = x;
-      }
+    for (int j = 0; j < 8; j++) {
+      const int lp = (ty * 8 + j) % tm.tp;
+      double x = 0.0;
+      for (int u = 0; u < tm.C; u++) x = fmax(x, sMax[u * tm.tp + lp]);
+      m[j] = x;
     }
     uint16_t *scd = c.scale + (size_t)op.dst_slot * c.slot_scale;
     double *dst = part + (size_t)op.dst_slot * c.slot_elems;
@@ -281,12 +275,7 @@ __global__ void __launch_bounds__(kThreadsG, 2)
         const int col = tx + 16 * q;
         if (col < kN) row[col] = o[j][q];
       }
-      if (tx == 0) {
-        if (SAFE)
-          scd[(size_t)p * tm.C + cat] = (uint16_t)s_out;
-        else if (cat == 0)
-          scd[p] = (uint16_t)s_out;
-      }
+      if (tx == 0 && cat == 0) scd[p] = (uint16_t)s_out;
     }
   }
 }
@@ -313,11 +302,6 @@ constexpr int kWarpsW = 8, kThreadsW = 32 * kWarpsW;
 constexpr size_t kSmemW = sizeof(double) * 3 * (size_t)kFrag;
 static_assert(kWarpsW * 8 == kRows, "a warp holds 8 patterns");
 
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 // element i of a matrix in fragment order, [16 K steps][4 pairs of N tiles][32 lanes][2]: its
 // contraction index k and output state x
 __device__ __forceinline__ void frag_place(int i, int &k, int &x) {
@@ -552,31 +536,27 @@ int g61_pattern_granule(const Session *s) {
 
 int launch_traverse_g61(Session *s, int nops, int p0, int p1) {
   if (nops <= 0 || p1 <= p0) return GEMS_OK;
-  const int tp = tile_patterns(s->desc.ncat);
   const bool safe = s->desc.scaling == GEMS_SCALE_SAFE;
-  const int gran = safe ? kRows : tp;
+  const int gran = g61_pattern_granule(s);
   if (p0 % gran != 0 || (p1 % gran != 0 && p1 != s->P)) {
     set_error("FP64 61-state traversal: pattern range not aligned to its pattern tiles");
     return GEMS_ERR_BAD_ARG;
   }
   cudaEvent_t ev0;
   if (int st = prof_begin(s, 0, &ev0)) return st;
-  const int tile0 = p0 / gran;
-  const int grid = (p1 + tp - 1) / tp - tile0;
+  const int tile0 = p0 / gran, tiles = (p1 + gran - 1) / gran - tile0;
   // the limit is a per-kernel attribute shared by every thread of the process: always the same
   // value
   if (safe) {  // FP64 tensor cores, one category per tile
-    const int g = ((p1 + kRows - 1) / kRows - tile0) * s->desc.ncat;
     GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61w, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kSmemW));
-    k_traverse_g61w<<<g, kThreadsW, kSmemW, s->stream>>>(s->ctx(), s->d_ops, nops, s->d_opmats,
-                                                         s->op_stride, tile0);
+    k_traverse_g61w<<<tiles * s->desc.ncat, kThreadsW, kSmemW, s->stream>>>(
+        s->ctx(), s->d_ops, nops, s->d_opmats, s->op_stride, tile0);
   } else {  // NORM: a pattern's categories in one tile, FP64 FMA
-    GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61<false>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemG));
-    k_traverse_g61<false><<<grid, kThreadsG, kSmemG, s->stream>>>(s->ctx(), s->d_ops, nops,
-                                                                   s->d_opmats, s->op_stride,
-                                                                   tile0);
+    GEMS_CUDA(cudaFuncSetAttribute(k_traverse_g61, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kSmemG));
+    k_traverse_g61<<<tiles, kThreadsG, kSmemG, s->stream>>>(s->ctx(), s->d_ops, nops, s->d_opmats,
+                                                            s->op_stride, tile0);
   }
   s->launches++;
   GEMS_CUDA(cudaGetLastError());

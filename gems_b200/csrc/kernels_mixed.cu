@@ -27,27 +27,6 @@ __device__ __forceinline__ float group_maxf(float v, int G) {
   for (int o = 1; o < G; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[32]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[k][w] = x;
-  }
-  __syncthreads();
-  if (w == 0) {
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      double x = lane < nw ? sh[k][lane] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      v[k] = x;
-    }
-  }
-  __syncthreads();
-}
-
 // P_c(t) for both children of every op (FP64 -> FP32), and tip tables P_c . indicator.
 // opmats (as float): [op][side][C][n][n] then [op][side][unknown+1][C][n]; grid (nops, 2).
 __global__ void k_prep_ops_mixed(DevCtx c, const DevOp *ops, float *opm, size_t stride_f) {
@@ -220,12 +199,6 @@ __global__ void __launch_bounds__(kThreads) k_traverse_mixed(DevCtx c, const Dev
 // blocks' sums in index order and writes them to pinned host memory.
 // ----------------------------------------------------------------------------------------
 constexpr int kWarpsL = 4;
-
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 template <int N, bool SAFE>
 __device__ __forceinline__ void theta_mixed(const DevCtx &c, const gems_branch &br, int nblocks,
@@ -418,7 +391,7 @@ int launch_traverse_mixed(Session *s, int nops, int p0, int p1) {
 
 // blocks of k_theta_mixed: at most one wave
 static int lift_blocks(const Session *s) {
-  return std::min(148 * (s->desc.nstates == 61 ? 3 : 5), (s->P / 8 + kWarpsL - 1) / kWarpsL);
+  return std::min(s->nsm * (s->desc.nstates == 61 ? 3 : 5), (s->P / 8 + kWarpsL - 1) / kWarpsL);
 }
 
 // theta (and optionally the branch lnL) from the two FP32 partials of br, 20 or 61 states
@@ -462,7 +435,7 @@ int enqueue_lnl_mixed_batch(Session *const *ss, const gems_branch *br, int n) {
     }
     // about one wave of blocks over all sessions: each block lays out its inv_evec once
     const int most = lift_blocks(s0);
-    const int per = std::min(most, std::max(1, 148 * (ns == 61 ? 3 : 5) / m));
+    const int per = std::min(most, std::max(1, s0->nsm * (ns == 61 ? 3 : 5) / m));
     cudaEvent_t ev0;
     if (int st = prof_begin(s0, 1, &ev0)) return st;
     fn<<<dim3(per, m), 32 * kWarpsL, smem, s0->stream>>>(b, most);

@@ -22,27 +22,6 @@ namespace {
 constexpr int kRellChunkLnl = 4096;   // patterns per CTA, lnL (16 KB of float terms)
 constexpr int kRellChunkDerv = 2048;  // patterns per CTA, derivatives (32 KB of double terms)
 
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[32]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[k][w] = x;
-  }
-  __syncthreads();
-  if (w == 0) {
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      double x = lane < nw ? sh[k][lane] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      v[k] = x;
-    }
-  }
-  __syncthreads();
-}
-
 constexpr int kRellThreads = 256;  // 8 warps
 constexpr int kRellRows = 32;      // replicate rows per CTA (4 per warp)
 

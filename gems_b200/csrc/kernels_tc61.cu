@@ -86,11 +86,6 @@ constexpr int kPrepThreads = 256;
 __host__ __device__ constexpr size_t prep61_smem_doubles(int C) {
   return (size_t)C * kNP + 2 * (size_t)kNP * kNP;
 }
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 __global__ void __launch_bounds__(kPrepThreads, 2)
     k_prep_ops_tc61(const __grid_constant__ TcJob one, const TcJob *__restrict__ jobs,
                     size_t stride_f) {

@@ -1666,13 +1666,12 @@ int traverse_v2_wave_patterns(const Session *s) {
   } else {
     fn = traverse_f20_kernel(s, s->P, &threads, &per_block);
   }
-  int nsm = 0, per_sm = 0;
-  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->desc.device) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  return per_sm * nsm * per_block;
+  return per_sm * s->nsm * per_block;
 }
 
 int traverse_v2_shape(const Session *s, int *patterns_per_group, int *blocks_per_sm) {

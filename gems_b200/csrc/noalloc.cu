@@ -54,27 +54,6 @@ struct ModelPack {
   double props[kMaxCat];
 };
 
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[32]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[k][w] = x;
-  }
-  __syncthreads();
-  if (w == 0) {
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      double x = lane < nw ? sh[k][lane] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      v[k] = x;
-    }
-  }
-  __syncthreads();
-}
-
 // per-CTA sums of freq * pattern lnL (raw, and with non-finite values clamped to
 // 4 log(2^-256)) into scratch[2 * blockIdx.x .. +1]
 __global__ void __launch_bounds__(kThreadsNa) k_lnl_theta_na(

@@ -448,7 +448,7 @@ int load_tips(Session *s, const uint8_t *src, size_t src_pitch, cudaMemcpyKind k
   GEMS_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned int), s->stream));
   GEMS_CUDA(cudaMemcpy2DAsync(s->d_tips, s->P, src, src_pitch, s->desc.nptn, s->desc.ntaxa, kind,
                               s->stream));
-  k_tips_max<<<148 * 8, 256, 0, s->stream>>>(s->d_tips, s->P, s->desc.nptn, s->desc.ntaxa, 0,
+  k_tips_max<<<s->nsm * 8, 256, 0, s->stream>>>(s->d_tips, s->P, s->desc.nptn, s->desc.ntaxa, 0,
                                              s->P, d_max);
   s->launches++;
   GEMS_CUDA(cudaGetLastError());
@@ -533,6 +533,9 @@ int gems_session_create(const gems_session_desc *desc, gems_session **out) {
     return code;
   };
   cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&s->nsm, cudaDevAttrMultiProcessorCount, desc->device)) !=
+      cudaSuccess)
+    return fail(e, "cudaDeviceGetAttribute");
 #define ALLOC(ptr, bytes)                                           \
   if ((e = cudaMalloc((void **)&(ptr), (bytes))) != cudaSuccess) \
     return fail(e, "cudaMalloc " #ptr);
@@ -1039,7 +1042,7 @@ int gems_branch_lnl_from_host(gems_session *s, const uint8_t *states, const doub
     GEMS_CUDA(cudaEventRecord(s->chunk_ev[c], cs));
     GEMS_CUDA(cudaStreamWaitEvent(ks, s->chunk_ev[c], 0));
     const long long words = (long long)(p1 - p0) / 16 * ntaxa;
-    const int grid = (int)std::min<long long>(148 * 8, (words + 255) / 256);
+    const int grid = (int)std::min<long long>(s->nsm * 8, (words + 255) / 256);
     k_tips_max<<<grid, 256, 0, ks>>>(s->d_tips, s->P, n, ntaxa, p0, p1, d_max);
     s->launches++;
     GEMS_CUDA(cudaGetLastError());
