@@ -433,7 +433,8 @@ class Session:
 
     def set_autotune(self, on=True, force_shape=None):
         """Tune the 4-state traversal's launch shape on its first large traversal (default), or
-        force shape k of the kernel's list (comparisons)."""
+        force shape k of the kernel's list (comparisons; op lists of branch calls then run as
+        traversals too)."""
         v = 2 + int(force_shape) if force_shape is not None else int(on)
         _check(self.lib.gems_session_set_option(self.handle, 3, v), "set_option")
 

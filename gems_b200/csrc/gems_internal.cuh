@@ -281,8 +281,8 @@ int cuda_status(cudaError_t e, const char *what);
 int launch_prep_ops(Session *s, int nops);
 // patterns [p0, p1) of the traversal, p1 <= P (every launch_traverse* below alike)
 int launch_traverse(Session *s, int nops, int p0, int p1);
-// branch terms (kernels_branch.cu).  theta_in_kernel: theta is formed by the kernel that uses it
-// (else launch it first: enqueue_theta_mixed); br null: theta as stored
+// branch terms (kernels_branch.cu, branch_kernels.cuh).  theta_in_kernel: theta is formed by the
+// kernel that uses it (else launch it first: enqueue_theta_mixed); br null: theta as stored
 bool theta_in_kernel(const Session *s);
 // whether a branch call runs these node updates in its own launch (`ops` of the calls below;
 // validated by the caller)
@@ -351,7 +351,7 @@ int launch_prep_ops_g61(Session *s, int nops);
 // p0 and p1 multiples of g61_pattern_granule (p1 may be P)
 int g61_pattern_granule(const Session *s);
 int launch_traverse_g61(Session *s, int nops, int p0, int p1);
-// the grid barrier's time-out path, run on purpose (kernels_fp64.cu)
+// the time-out paths of the Newton loop's waits, run on purpose (kernels_branch.cu)
 int check_barrier_timeout(int device, int *status);
 // bootstrap reweighting (kernels_rell.cu)
 // scratch of the tiled reductions (per replicate row and pattern chunk), in doubles

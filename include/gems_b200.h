@@ -122,8 +122,9 @@ enum { GEMS_OPT_TENSOR_CORES = 1, GEMS_OPT_TILED_FP64 = 2, GEMS_OPT_AUTOTUNE = 3
  * scaling, categories, pattern count to the power of two) with at least 2^22 pattern-updates
  * times every launch shape of the traversal kernel (patterns per lane group x blocks per SM; all
  * give the same values) and keeps the fastest for the process; 0 keeps the default shape (or
- * the one already chosen for the class); 2 + k forces shape k (for comparisons).  No
- * counterpart in the reference.  gems_session_traversal_shape reports the shape in use and
+ * the one already chosen for the class); 2 + k forces shape k (for comparisons: every op list of
+ * the session then runs as a traversal of that shape, those of branch calls too).  Lists that write
+ * a slot after reading it are not tuned on.  No counterpart in the reference.  gems_session_traversal_shape reports the shape in use and
  * whether it was tuned (0 0 0 for the forms that have one shape). */
 int gems_session_traversal_shape(gems_session *s, int *patterns_per_group, int *blocks_per_sm,
                                  int *tuned);
