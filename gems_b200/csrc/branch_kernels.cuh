@@ -773,7 +773,9 @@ __global__ void __launch_bounds__(HELD ? newton_threads(E2) : stream_threads(E2)
   const long per = nt / L, step = per * gridDim.x;
   const long b0 = (long)blockIdx.x * per;
   const int sub = threadIdx.x / L;
-  const uint32_t s_bars = tc::sptr(&bars[0]);
+  // (this block's receive address is kept, not made in each evaluation: mixed, 4 states, 8 categories,
+  // 250,000 patterns 87.4 us a loop of one evaluation instead of 94.5)
+  const uint32_t s_recv = tc::sptr(&recv[0][0]), s_bars = tc::sptr(&bars[0]);
   const uint32_t expect = CS * nw * sizeof(double2);
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; i++) {
@@ -785,10 +787,10 @@ __global__ void __launch_bounds__(HELD ? newton_threads(E2) : stream_threads(E2)
   // the others' barriers are ready once all blocks have been here (waited for below)
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
-  double *small = tab + 3 * len;
+  const double *small = tab + 3 * len;
   if constexpr (small_form<SRC, E2>())
     if (ops.n) {
-      small_tables<SRC>(c, ops, small);
+      small_tables<SRC>(c, ops, tab + 3 * len);
       __syncthreads();
     }
   auto updates = [&](const long (&p)[2]) {
@@ -907,8 +909,8 @@ __global__ void __launch_bounds__(HELD ? newton_threads(E2) : stream_threads(E2)
     nevals++;
     const uint32_t bar = s_bars + 8 * set;
     if (lane < CS)
-      send_pair(cluster_addr(tc::sptr(&recv[set][rank * nw + warp]), lane), cluster_addr(bar, lane),
-                v0, v1);
+      send_pair(cluster_addr(s_recv + (set * kMaxCluster * nw + rank * nw + warp) * 16, lane),
+                cluster_addr(bar, lane), v0, v1);
     bool ok = cluster_wait(bar, use);
     v0 = v1 = 0.0;
     if (ok)
