@@ -1,5 +1,5 @@
-// branch_kernels.cuh -- the kernels of the branch terms: log-likelihood, theta, derivatives, lnL from theta, and
-// the Newton loop on the device (phylokernelnew.h:2053-3495, utils/optimization.cpp:422-499).
+// branch_kernels.cuh -- the kernels of the branch terms: log-likelihood, theta, derivatives, lnL from
+// theta, and the Newton loop on the device (phylokernelnew.h:2053-3495, utils/optimization.cpp:422-499).
 //
 // Every term is a dot product over the C * n elements of a pattern's theta = node (*) dad (eigen
 // space) with tables of exp(eval_i r_c t):
